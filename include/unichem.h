@@ -311,7 +311,7 @@ int uc_profile_read(uc_ctx *ctx, double *ms, int *launches);
  *                         (UNICHEM_UPDATE=inplace), 2 per pass with two Y sets
  *                         (UNICHEM_UPDATE=twoset), chosen at uc_init
  *   "update_chunk"        passes per chunk of the tile-resident update (UNICHEM_TR_CHUNK, 16)
- *   "update_lockstep"     1 if its warps run species by species in step (UNICHEM_TR_LOCKSTEP)
+ *   "update_lockstep"     UNICHEM_TR_LOCKSTEP as given (no effect: a tile's warps are always in step)
  *   "update_flops_per_cell_pass"  floating-point operations of one cell and pass of the
  *                         update (each multiplication, addition and division one)
  *   "update_ip_warps"     warps per CTA of the species update with Y in place

@@ -50,8 +50,8 @@ __device__ __forceinline__ double gibbs_exp(const double *a, double ELOGT, doubl
     double TKD2 = TKD * TKD / 6.0;
     double TKD3 = TKD1 * TKD2;
     double TKD4 = (double)1.2f * TKD1 * TKD3;
-    double g0 = a[0] * (ELOGT - 1.0) + a[1] * TKD1 + a[2] * TKD2 + a[3] * TKD3 + a[4] * TKD4 - a[5] / TKD + a[6];
-    return exp(g0);
+    const double g0 = __fma_rn(a[4], TKD4, __fma_rn(a[3], TKD3, __fma_rn(a[2], TKD2, __fma_rn(a[1], TKD1, __dmul_rn(a[0], ELOGT - 1.0)))));
+    return exp(g0 - a[5] / TKD + a[6]);
 }
 
 // Phases 1b-1c of a tile: TBODY from the Y/W rows left in sRC by phase 1a, the
@@ -163,8 +163,8 @@ __device__ __forceinline__ void tile_rates_fp64(const DevParams &P, const PairTa
                 if (T.troe[0] > 0.0) {
                     double FCLOG;
                     if (T.troe[1] == 0.0) FCLOG = log10(T.troe[0]);
-                    else FCLOG = log10((1.0 - T.troe[0]) * exp(-(TKD / T.troe[1])) +
-                                       T.troe[0] * exp(-(TKD / T.troe[2])) + exp(-(T.troe[3] / TKD)));
+                    else FCLOG = log10(__fma_rn(T.troe[0], exp(-(TKD / T.troe[2])),
+                                                __dmul_rn(1.0 - T.troe[0], exp(-(TKD / T.troe[1])))) + exp(-(T.troe[3] / TKD)));
                     const double CPLOG = log10(AK0M) - ((double)0.4f + (double)0.67f * FCLOG);
                     const double z = CPLOG / ((double)0.75f - (double)1.27f * FCLOG - (double)0.14f * CPLOG);
                     RFACT = pow(10.0, FCLOG / (1.0 + z * z));

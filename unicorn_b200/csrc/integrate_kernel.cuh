@@ -17,13 +17,14 @@
 // Per tile the CTA keeps everything on chip: the reaction-pair table (one
 // bulk copy per CTA), the tile's RC plane [544][32], Y, Y at the sub-step
 // start and the update's scratch. The rates of a sub-step run on all NW
-// warps (the phases of chem_fp64_kernel); the update program, the closure
-// and the Newton for T run on warp 0 (lane = cell) with RC read from shared
-// memory.
+// warps (the phases of chem_fp64_kernel). The update runs on three of them, with
+// the program of the tile-resident update (two form the species' sums, warp 0
+// closes them; the two forms of the integration thus compute a cell the same way) and
+// RC and Y in shared memory; the closure and the Newton for T run on warp 0 (lane = cell).
 #pragma once
 #include "chem_kernel.cuh"
 #include "chem_mixed_kernel.cuh"
-#include "generated/update_program.cuh"
+#include "update_tr_kernel.cuh"
 
 namespace uc {
 
@@ -156,7 +157,8 @@ __device__ __forceinline__ double enthalpy_total(const DevParams &P, double tk, 
 }
 
 // Newton for T at total enthalpy ENTH (solveh.f:1186-1234). Returns tk;
-// sets *conv to false if 100 iterations did not meet the step tolerance.
+// sets *conv to false if 100 iterations did not meet the step tolerance. The multiply-adds are written out: a sum
+// of two products may be contracted either way, and the two forms of the integration compute a cell alike.
 __device__ __forceinline__ double temperature_at(const DevParams &P, double tk, const double *y, int ys, double ENTH,
                                                  bool *conv)
 {
@@ -187,8 +189,9 @@ __device__ __forceinline__ double temperature_at(const DevParams &P, double tk, 
     }
     *conv = false;
     for (int it = 1; it <= 100; ++it) {
-        const double DTKD = ((A1 + (A2 + (A3 + (A4 + A5 * TKD) * TKD) * TKD) * TKD) * TKD + A6 - ENTH * P.WMSTR / P.GASC) /
-                            (A1 + (2.0 * A2 + (3.0 * A3 + (4.0 * A4 + 5.0 * A5 * TKD) * TKD) * TKD) * TKD);
+        const double num = __fma_rn(__fma_rn(__fma_rn(__fma_rn(__fma_rn(A5, TKD, A4), TKD, A3), TKD, A2), TKD, A1), TKD, A6);
+        const double den = __fma_rn(__fma_rn(__fma_rn(__fma_rn(5.0 * A5, TKD, 4.0 * A4), TKD, 3.0 * A3), TKD, 2.0 * A2), TKD, A1);
+        const double DTKD = (num - ENTH * P.WMSTR / P.GASC) / den;
         if (fabs(DTKD) <= (double)0.001f) { *conv = true; break; }
         TKD = TKD - DTKD;
     }
@@ -448,6 +451,118 @@ __global__ void scatter_state_kernel(int n, int npad, RoundState s, double *y, d
     }
 }
 
+// A pass of the tile's update with RC and Y in shared memory (the warps of one tile as in update_tr_kernel:
+// two sum, one closes; see there). The closing warp writes species k while the others sum species k + 1,
+// which reads neither value of k but through the copies YOS.
+struct IntTile {
+    const double *rc;              // [544][32] at the lane's column, and so the others
+    double *y;                     // [52][32]
+    const double *ry0;             // [52][32]: rho * Y at the sub-step start
+    double *part;                  // [slots][32] pairs
+    const double *sour;            // [6][32]
+    int *flag;
+};
+// the kernel's dynamic shared memory, laid out in this order
+constexpr size_t INT_OFF_RC = PAIRTAB_BYTES, INT_OFF_Y = INT_OFF_RC + sizeof(double) * LRX * TILE,
+                 INT_OFF_G = INT_OFF_Y + sizeof(double) * LSP * TILE, INT_OFF_Y0 = INT_OFF_G + sizeof(double) * LSP * TILE,
+                 INT_OFF_C = INT_OFF_Y0 + sizeof(double) * LSP * TILE, INT_OFF_S = INT_OFF_C + sizeof(double) * SC_N * TILE,
+                 INT_OFF_BAR = INT_OFF_S + sizeof(double) * 6 * TILE, INT_OFF_QUIT = INT_OFF_BAR + 8;
+static_assert(INT_OFF_QUIT + 8 <= INT_SMEM, "shared memory of the integrator");
+static_assert(2 * UC_CO_SLOTS <= LSP, "the partial sums take the place of the Gibbs functions");
+// from the shared array itself, so that a function that is not inlined reads it with shared-memory loads
+__device__ __forceinline__ IntTile int_tile()
+{
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int lane = threadIdx.x & 31;
+    return {reinterpret_cast<double *>(smem + INT_OFF_RC) + lane, reinterpret_cast<double *>(smem + INT_OFF_Y) + lane,
+            reinterpret_cast<double *>(smem + INT_OFF_Y0) + lane, reinterpret_cast<double *>(smem + INT_OFF_G) + 2 * lane,
+            reinterpret_cast<double *>(smem + INT_OFF_S) + lane, reinterpret_cast<int *>(smem + INT_OFF_QUIT)};
+}
+#define CO_WAIT_Y(set) asm volatile("bar.sync %0, 96;" ::"n"(1 + (set)) : "memory")
+#define CO_ARRIVE_Y(set) asm volatile("bar.arrive %0, 96;" ::"n"(1 + (set)) : "memory")
+#define CO_WAIT_P(set) asm volatile("bar.sync %0, 96;" ::"n"(3 + (set)) : "memory")
+#define CO_ARRIVE_P(set) asm volatile("bar.arrive %0, 96;" ::"n"(3 + (set)) : "memory")
+#define YO(k) t.y[(k) * TILE]
+#define YOS(m) ysh[m]
+#define SOUR(m) t.sour[(m) * TILE]
+#define RCS2(i) make_double2(t.rc[(UC_CO_NT + 2 * (i)) * TILE], t.rc[(UC_CO_NT + 2 * (i) + 1) * TILE])
+#define TM_LD2(b, q, col, p)                                    \
+    do {                                                        \
+        bank##b[2 * (q)] = t.rc[2 * (p) * TILE];                \
+        bank##b[2 * (q) + 1] = t.rc[(2 * (p) + 1) * TILE];      \
+    } while (0)
+#define TM_LD4(b, q, col, p0, p1)       \
+    do {                                \
+        TM_LD2(b, q, col, p0);          \
+        TM_LD2(b, (q) + 1, col, p1);    \
+    } while (0)
+#define TM_LD8(b, q, col, p0, p1, p2, p3)     \
+    do {                                      \
+        TM_LD4(b, q, col, p0, p1);            \
+        TM_LD4(b, (q) + 2, col, p2, p3);      \
+    } while (0)
+#define TM_WAIT(b, n) do { } while (0)
+#define RCT(b, i) bank##b[i]
+#define CO_PUT(slot, a, b) co_st2(t.part + (slot) * (2 * TILE), a, b)
+#define CO_GET(buf, k, mine, now) do { } while (0)
+#define CO_CHECK()                                              \
+    do {                                                        \
+        asm volatile("bar.sync 5, 96;" ::: "memory");          \
+        if (co_ldi(t.flag)) return false;                       \
+    } while (0)
+template <int W>
+__device__ __noinline__ bool int_sums()
+{
+    const IntTile t = int_tile();
+    double ysh[UC_CO_NSHADOW], bank0[2 * UC_CO_SEG], bank1[2 * UC_CO_SEG];
+    if (W == 0) UC_CO_SUMS_0();
+    else UC_CO_SUMS_1();
+    return true;
+}
+#define CO_TAKE(slot, a, b) co_ld2(t.part + (slot) * (2 * TILE), a, b)
+#define CO_QUOT(n, d) co_quot(n, d)
+#define CO_GIVE(buf, k) do { } while (0)
+#define RY0(k) t.ry0[(k) * TILE]
+#define DTW(k) (dt * prm.WM[k])
+#define CO_PF(s, k) do { } while (0)
+#define FSS(s) 0.0
+#define FNS(s) 0.0
+#define CO_TAIL(k) do { if (fnew < 0.0) fnew = 0.0; if (!done) t.y[(k) * TILE] = fnew; } while (0)
+__device__ __noinline__ bool int_close(const DevParams &prm, double rho, double dt, double sor1, double sor2,
+                                       bool done, double &rsd)
+{
+    const IntTile t = int_tile();
+    UC_CO_CLOSE();
+    return true;
+}
+// before the first pass: the last run's values stand in shared memory already
+__device__ __forceinline__ void int_close_begin() { CO_ARRIVE_Y(UC_CO_LAST_SET); }
+#undef CO_WAIT_Y
+#undef CO_ARRIVE_Y
+#undef CO_WAIT_P
+#undef CO_ARRIVE_P
+#undef CO_QUOT
+#undef YO
+#undef YOS
+#undef SOUR
+#undef RCS2
+#undef TM_LD2
+#undef TM_LD4
+#undef TM_LD8
+#undef TM_WAIT
+#undef RCT
+#undef CO_PUT
+#undef CO_GET
+#undef CO_CHECK
+#undef CO_TAKE
+#undef CO_GIVE
+#undef RY0
+#undef DTW
+#undef CO_PF
+#undef FSS
+#undef FNS
+#undef CO_TAIL
+
 // MIXED: the rates of every sub-step in the mixed form (tile_rates_mixed; a tile with a rate beyond the
 // FP32 range is recomputed in FP64), the update, closure and Newton in FP64 as in the FP64 form.
 template <int NW, bool MIXED>
@@ -455,13 +570,14 @@ __global__ void __launch_bounds__(NW * 32, 1) integrate_fp64_kernel(const IntArg
 {
     extern __shared__ __align__(128) unsigned char smem[];
     PairTab *sTab = reinterpret_cast<PairTab *>(smem);
-    double *sRC = reinterpret_cast<double *>(smem + PAIRTAB_BYTES);   // [544][32]
-    double *sY = sRC + LRX * TILE;                                    // [52][32] current Y (YO)
-    double *sYN = sY + LSP * TILE;                                    // [52][32] Gibbs scratch / YN
-    double *sY0 = sYN + LSP * TILE;                                   // [52][32] Y at the sub-step start
-    double *sC = sY0 + LSP * TILE;                                    // [SC_N][32]
-    double *sS = sC + SC_N * TILE;                                    // [6][32] soot sources
-    uint64_t *bar = reinterpret_cast<uint64_t *>(sS + 6 * TILE);
+    double *sRC = reinterpret_cast<double *>(smem + INT_OFF_RC);      // [544][32]
+    double *sY = reinterpret_cast<double *>(smem + INT_OFF_Y);        // [52][32] current Y
+    double *sYN = reinterpret_cast<double *>(smem + INT_OFF_G);       // [52][32] Gibbs scratch / partial sums
+    double *sY0 = reinterpret_cast<double *>(smem + INT_OFF_Y0);      // [52][32] rho * Y at the sub-step start
+    double *sC = reinterpret_cast<double *>(smem + INT_OFF_C);        // [SC_N][32]
+    double *sS = reinterpret_cast<double *>(smem + INT_OFF_S);        // [6][32] soot sources
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + INT_OFF_BAR);
+    int *s_quit = reinterpret_cast<int *>(smem + INT_OFF_QUIT);       // no more passes of this sub-step
     __shared__ int s_tile, s_smax;
     const DevParams &P = *a.P;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -534,62 +650,35 @@ __global__ void __launch_bounds__(NW * 32, 1) integrate_fp64_kernel(const IntArg
             if (!MIXED || tile_rates_mixed<NW>(P, a.tabm, sRC, sY, sYN, sC, sS, TILE, lane, lane, warp))
                 tile_rates_fp64<NW>(P, sTab, sRC, sY, sYN, sC, sS, TILE, lane, lane, warp);
             __syncthreads();
-            if (warp == 0 && st < ns) {
+            if (warp == 1) { while (int_sums<0>()) {} }
+            else if (warp == 2) { while (int_sums<1>()) {} }
+            else if (warp == 0) {
                 const double dt = a.dt / (double)ns;
                 double so[6];
 #pragma unroll
                 for (int m = 0; m < 6; ++m) so[m] = sS[m * TILE + lane];
-                for (int k = 0; k < LSP; ++k) sY0[k * TILE + lane] = sY[k * TILE + lane];
+                for (int k = 0; k < LSP - 1; ++k) sY0[k * TILE + lane] = rho * sY[k * TILE + lane];
                 const double s10 = s1, s20 = s2;
-                for (int pass = 1; pass <= a.isor; ++pass) {
+                bool done = st >= ns;
+                int_close_begin();
+                for (int pass = 1;; ++pass) {
+                    const int quit = pass > a.isor || __all_sync(0xffffffffu, done);
+                    if (lane == 0) *s_quit = quit;
                     double rsd = 0.0;
-                    // Shared-memory operands; the empty asm with a memory clobber before each
-                    // species block keeps the compiler from hoisting loads across blocks (it
-                    // runs out of registers otherwise), while loads within a block still overlap.
-#define YO(k) sY[(k) * TILE + lane]
-#define YN(k) sYN[(k) * TILE + lane]
-#define Y0(k) sY0[(k) * TILE + lane]
-#define RC(r) sRC[(r) * TILE + lane]
-#define RC_LAST(r) sRC[(r) * TILE + lane]
-#define SOUR(m) so[m]
-#define WM(k) P.WM[k]
-#define FACE_SUM(k) 0.0
-#define FACE_NBR(k) 0.0
-#define UC_UPDATE_TAIL(k) do { if (fnew < 0.0) fnew = 0.0; sYN[(k) * TILE + lane] = fnew; } while (0)
-#define UC_UPDATE_SYNC() do { } while (0)
-#define UC_UPDATE_BLOCK_BEGIN(b) asm volatile("" ::: "memory")
-                    UC_UPDATE_PROGRAM();
-#undef YO
-#undef YN
-#undef Y0
-#undef RC
-#undef RC_LAST
-#undef SOUR
-#undef WM
-#undef FACE_SUM
-#undef FACE_NBR
-#undef UC_UPDATE_TAIL
-#undef UC_UPDATE_SYNC
-#undef UC_UPDATE_BLOCK_BEGIN
-                    // soot mass fraction and number density (solvesp.f:2807-2832)
-                    const double y2 = sYN[1 * TILE + lane], y4 = sYN[3 * TILE + lane], y5 = sYN[4 * TILE + lane];
-                    const double y22 = sYN[21 * TILE + lane];
-                    double rhs1 = rho * s10 + dt * ((double)0.012011f / P.WMSTR) *
-                                                  (2.0 * so[0] * y22 - so[2] * y2 - so[3] * y5 - so[4] * y4);
-                    double fnew = sor2 * s1 + rhs1 * sor1 / ((rho - 0.0) - 0.0);
-                    rsd += fabs(s1 - fnew);
-                    if (fnew < 0.0) fnew = 0.0;
-                    const double n1 = fnew;
-                    rhs1 = rho * s20 + dt * so[1] * y22;
-                    const double rhs2 = -(dt * so[5]);
-                    fnew = sor2 * s2 + rhs1 * sor1 / ((rho - 0.0) - rhs2);
-                    if (fnew < 0.0) fnew = 0.0;
-                    for (int k = 0; k < LSP - 1; ++k) sY[k * TILE + lane] = sYN[k * TILE + lane];
-                    s1 = n1;
-                    s2 = fnew;
-                    ++npass;
-                    if (rsd / (double)(LSP - 1) <= a.tol) break;
+                    if (!int_close(P, rho, dt, sor1, sor2, done, rsd)) break;
+                    double ys[22], n1, n2;
+                    ys[1] = sY[1 * TILE + lane]; ys[3] = sY[3 * TILE + lane];
+                    ys[4] = sY[4 * TILE + lane]; ys[21] = sY[21 * TILE + lane];
+                    co_soot(ys, so, s10, s20, rho, dt, P.WMSTR, sor1, sor2, s1, s2, n1, n2, rsd);
+                    if (!done) {
+                        s1 = n1;
+                        s2 = n2;
+                        ++npass;
+                        if (rsd / (double)(LSP - 1) <= a.tol) done = true;
+                    }
                 }
+            }
+            if (warp == 0 && st < ns) {
                 // N2 closure and renormalisation (solvesp.f:2839-2915)
                 double ft = sY[lane];
                 for (int k = 1; k < LSP - 1; ++k) ft = ft + sY[k * TILE + lane];

@@ -73,10 +73,9 @@ struct uc_ctx {
     bool tr_adapt = true;              // ... longer while the last call's pass count says more are to come
                                        // (off when UNICHEM_TR_CHUNK fixes the chunk, or when the snapshots
     bool tr_adapt_nomem = false;       // of the longer chunks did not fit in device memory)
-    bool tr_lock = false;              // ... with the warps of a block in step species by species
-                                       // (measured on 1M cells, 100 passes: 227 ms in step, 221 ms free)
+    bool tr_lock = false;              // UNICHEM_TR_LOCKSTEP as given: no effect (a tile's warps are in step)
     double *tr_snap = nullptr, *tr_partial = nullptr;
-    CUtensorMap tr_map[2];             // the RC plane as a 2-D tensor [544][npad], boxes of 256 and 144 rows
+    CUtensorMap tr_map[2];             // the RC plane as a 2-D tensor [544][npad], boxes of 168 and 208 rows
     const double *tr_map_base = nullptr;
     size_t tr_snap_cap = 0;
     // species-equation faces assembled on the device (grid, flow, coefficients)
@@ -530,11 +529,10 @@ static int encode_rc_map(uc_ctx *ctx)
     return UC_OK;
 }
 
-// the tile-resident update kernel for the face terms given or not, warps in step or not
-static const void *tr_kernel(bool faces, bool lock)
+// the tile-resident update kernel for the face terms given or not
+static const void *tr_kernel(bool faces)
 {
-    if (faces) return lock ? (const void *)update_tr_kernel<true, true> : (const void *)update_tr_kernel<true, false>;
-    return lock ? (const void *)update_tr_kernel<false, true> : (const void *)update_tr_kernel<false, false>;
+    return faces ? (const void *)update_tr_kernel<true> : (const void *)update_tr_kernel<false>;
 }
 
 #define RET_IF(x)                 \
@@ -630,7 +628,7 @@ extern "C" int uc_init(const uc_inputs *in, int ncell, int device, uc_ctx **out)
         if (ctx->upd_kind == 0) {
             if (const char *k = getenv("UNICHEM_TR_LOCKSTEP")) ctx->tr_lock = atoi(k) != 0;
             for (int f = 0; f < 2 && e == cudaSuccess; ++f) {
-                const void *fn = tr_kernel(f != 0, ctx->tr_lock);
+                const void *fn = tr_kernel(f != 0);
                 e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TR_SMEM);
                 int tr_per_sm = 0;
                 if (e == cudaSuccess) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&tr_per_sm, fn, TR_WARPS * 32, TR_SMEM);
@@ -1088,7 +1086,7 @@ extern "C" int uc_species_update(uc_ctx *ctx, double dt, int isor, double relx, 
         RET_IF(encode_rc_map(ctx));
         void *targs[] = {&a, &t, &ctx->tr_map[0], &ctx->tr_map[1]};
         prof_begin(ctx, UC_K_UPDATE, slot);
-        CK(cudaLaunchCooperativeKernel(tr_kernel(fs != nullptr || fn != nullptr, ctx->tr_lock), dim3(ctx->nsm),
+        CK(cudaLaunchCooperativeKernel(tr_kernel(fs != nullptr || fn != nullptr), dim3(ctx->nsm),
                                        dim3(TR_WARPS * 32), targs, TR_SMEM, ctx->stream));
         prof_end(ctx, slot);
         if (passes) {

@@ -398,6 +398,644 @@ def gen_tr_program(blocks, uses: dict, shadow: list[int]) -> str:
     return "\n".join(L) + "\n"
 
 
+# ------------------------------------------------------------------ grouped form, three warps per tile
+
+CO_NT, CO_PIECE = 336, 168       # rows in tensor memory, staged in pieces of CO_PIECE rows
+CO_PAIRS = (20, 64)              # row pairs of each piece that each of the summing warps holds
+CO_SHARE = (0.40, 0.60)          # of the work (the first ones of an SM's three tiles run on one scheduler)
+CO_SUMS = len(CO_PAIRS)
+CO_SEG = 4                       # row pairs per register bank of tensor-memory operands
+CO_REUSE = 10                    # statements over which a row pair read from shared memory stays in registers
+CO_LAST = 48                     # the last species whose sums have terms (argon and helium follow)
+CO_LONG = 6                      # terms from which a sum has two accumulators
+CO_NEWSUM = 4.0                  # see _share_out
+CO_RUN, CO_VALUES = 3, 7         # species closed in one step, and the partial sums a warp hands over for them
+
+
+def _grouped_sums(blocks):
+    """Per species block the terms of (production and extra, loss) as (coefficient, operand, Y leaves): the
+    operand is ("RC", r), ("SOUR", m) or None. Terms that are the literal zero are dropped."""
+    out = []
+    for b in blocks:
+        d = []
+        for keys in (("prod", "extra"), ("loss",)):
+            ts = []
+            for key in keys:
+                for s, t in b[key] or []:
+                    coef, op, ys = float(s), None, []
+                    for x in leaves(t, []):
+                        if x.kind == "num":
+                            coef *= x.val
+                        elif x.kind in ("RC", "SOUR"):
+                            assert op is None
+                            op = (x.kind, x.idx)
+                        else:
+                            assert x.kind in ("yo", "yn"), x.kind
+                            ys.append((x.kind, x.idx))
+                    if op is None and not ys and coef == 0.0:
+                        continue
+                    ts.append((coef, op, ys))
+            d.append(ts)
+        out.append(d)
+    return out
+
+
+def _pair(t):
+    return t[1][1] // 2 if t[1] is not None and t[1][0] == "RC" else -1
+
+
+def _runs(sums):
+    """The species in runs that are closed together: no species of a run is a factor, with its new value, of
+    another's sums in the same run. The fewest runs (an even number, so that the two sets of exchange buffers
+    alternate over the passes), at most CO_RUN species and CO_VALUES partial sums each."""
+    nb = CO_LAST + 1
+    dep = [{y[1] for side in sums[b] for _, _, ys in side for y in ys if y[0] == "yn"} for b in range(nb)]
+    best = {(0, 0, 0): (0, None)}                      # (species done, length of the last run, parity)
+    for e in range(1, nb + 1):
+        for m in range(1, min(CO_RUN, e) + 1):
+            run = range(e - m, e)
+            if any(dep[b] & set(run) for b in run):
+                continue
+            for m0 in range(CO_RUN + 1):
+                for par in range(2):
+                    if (e - m, m0, par) not in best:
+                        continue
+                    if len(_values(sums, run, range(e - m - m0, e - m))) > CO_VALUES:
+                        continue
+                    n = best[(e - m, m0, par)][0] + 1
+                    if n < best.get((e, m, 1 - par), (10 ** 9,))[0]:
+                        best[(e, m, 1 - par)] = (n, (e - m, m0, par))
+    at = min(((nb, m, 0) for m in range(1, CO_RUN + 1) if (nb, m, 0) in best), key=lambda k: best[k][0])
+    out = []
+    while at[0]:
+        out.append(list(range(at[0] - at[1], at[0])))
+        at = best[at][1]
+    return out[::-1]
+
+
+def _values(sums, run, prev):
+    """The partial sums of a run: (species, 'P' or 'L', factor of the run before or None)."""
+    out = []
+    for b in run:
+        for side, nm in enumerate("PL"):
+            ks = sorted({y[1] for _, _, ys in sums[b][side] for y in ys if y[0] == "yn" and y[1] in prev})
+            out += [(b, nm, None)] + [(b, nm, k) for k in ks]
+    return out
+
+
+def _pair(t):
+    return t[1][1] // 2
+
+
+def _share_out(sums, runs):
+    """Which of the summing warps takes which row pair of each run. A pair in tensor memory belongs to
+    one warp; a pair in shared memory may be read by any. The measure is the sum over the runs of the
+    largest share, since the warps meet after every run; found by a descent over swaps of tensor-memory
+    pairs from a fixed start."""
+    import random
+    ntp, nr = CO_NT // 2, len(runs)
+    cost = [dict() for _ in range(nr)]                # per run: pair -> statements and loads
+    for r, run in enumerate(runs):
+        for b in run:
+            for side in sums[b]:
+                for t in side:
+                    p = _pair(t)
+                    cost[r][p] = cost[r].get(p, 1.0) + 1.0 + 0.3 * max(0, len(t[2]) - 1)
+    where = [[(r, cost[r][p]) for r in range(nr) if p in cost[r]] for p in range(ntp)]
+    free = [sum(c for p, c in cost[r].items() if p >= ntp) for r in range(nr)]
+
+    def level(load, r):
+        """Time of run r, by the slowest warp, with the free pairs dealt out evenly."""
+        return max(sum(load[r]) + free[r], *[x / f for x, f in zip(load[r], CO_SHARE)])
+
+    owner, load = [0] * ntp, [[0.0] * CO_SUMS for _ in range(nr)]
+    for piece in range(CO_NT // CO_PIECE):
+        lo = piece * CO_PIECE // 2
+        left = list(CO_PAIRS)
+        for p in sorted(range(lo, lo + CO_PIECE // 2), key=lambda p: -sum(c for _, c in where[p])):
+            w = min((w for w in range(CO_SUMS) if left[w]),
+                    key=lambda w: (sum(max(0.0, load[r][w] + c - max(load[r])) for r, c in where[p]), -left[w]))
+            owner[p] = w
+            left[w] -= 1
+            for r, c in where[p]:
+                load[r][w] += c
+    rng = random.Random(1)
+    for _ in range(60000):
+        p = rng.randrange(ntp)
+        q = p // (CO_PIECE // 2) * (CO_PIECE // 2) + rng.randrange(CO_PIECE // 2)
+        if owner[p] == owner[q]:
+            continue
+        touched = sorted({r for r, _ in where[p]} | {r for r, _ in where[q]})
+        before = sum(level(load, r) for r in touched)
+
+        def swap():
+            for r, c in where[p]:
+                load[r][owner[p]] -= c
+                load[r][owner[q]] += c
+            for r, c in where[q]:
+                load[r][owner[q]] -= c
+                load[r][owner[p]] += c
+            owner[p], owner[q] = owner[q], owner[p]
+        swap()
+        if sum(level(load, r) for r in touched) > before + 1e-9:
+            swap()
+    # the free pairs: onto the least loaded warp, where a partial sum that the warp does not form yet counts as
+    # CO_NEWSUM statements (it has to be handed over and read)
+    share = []                                         # per run: pair -> warp
+    for r, run in enumerate(runs):
+        prev = set(runs[r - 1]) if r else set()
+        keys: dict = {}
+        for b in run:
+            for side, nm in enumerate("PL"):
+                for t in sums[b][side]:
+                    f = [y[1] for y in t[2] if y[0] == "yn" and y[1] in prev]
+                    keys.setdefault(_pair(t), set()).add((b, nm, f[0] if f else None))
+        mine = {p: owner[p] for p in cost[r] if p < ntp}
+        has = [set().union(*[keys[p] for p in mine if mine[p] == w]) for w in range(CO_SUMS)]
+        now = list(load[r])
+        for p in sorted((p for p in cost[r] if p >= ntp), key=lambda p: (-cost[r][p], p)):
+            w = min(range(CO_SUMS), key=lambda w: (now[w] + cost[r][p] + CO_NEWSUM * len(keys[p] - has[w])) / CO_SHARE[w])
+            mine[p] = w
+            has[w] |= keys[p]
+            now[w] += cost[r][p]
+        share.append(mine)
+    return owner, share
+
+
+def _added(parts) -> str:
+    """The sum of the parts from left to right, as CO_ADD."""
+    e = parts[0]
+    for x in parts[1:]:
+        e = f"CO_ADD({e}, {x})"
+    return e
+
+
+class _COEmit:
+    """Statements of one summing warp. RC(r) is the token @r@, bound later."""
+
+    def __init__(self, place=None):
+        self.updated: set[int] = set()
+        self.shadow: list[int] = []
+        self.place = place or {}           # pair -> tensor-memory column: pairs that are loaded together side by side
+
+    def key(self, t):
+        p = _pair(t)
+        return (0, self.place[p]) if p in self.place else (1, p)
+
+    def y(self, leaf) -> str:
+        kind, k = leaf
+        if kind == "yo" and k in self.updated:
+            if k not in self.shadow:
+                self.shadow.append(k)
+            return f"YOS({self.shadow.index(k)})"
+        return f"YO({k})"
+
+    def product(self, coef, op, ys) -> tuple:
+        """coef * op * ys as two factors (the second None where there is one)."""
+        parts = [self.y(v) for v in ys]
+        if op is not None:
+            parts.append(f"@{op[1]}@" if op[0] == "RC" else f"SOUR({op[1]})")
+        if coef != 1.0:
+            parts.insert(0, repr(coef))
+        e = parts[0]
+        for x in parts[1:-1]:
+            e = f"({e} * {x})"
+        return (e, None) if len(parts) == 1 else (e, parts[-1])
+
+    def sums(self, b, prod, loss, prev, fresh):
+        """Statements that form, of the given terms of species b, P and L (without the species of `prev`, the
+        run being closed, whose new values are not known yet) and what each species of prev multiplies in
+        them. `fresh`: the run before that, whose values arrive meanwhile. Returns the statements that need
+        no fresh value, those that do, and {(b, 'P' or 'L', factor or None): expression}."""
+        pre: list[tuple] = []              # (accumulator, its sum's number, addend)
+        post: list[tuple] = []
+        turn: dict[str, int] = {}
+        number = [0]
+
+        def add(st, var, expr, sum_=0):
+            st.append((var, sum_, expr))
+
+        # two accumulators, in turn, for a sum long enough that its chain of additions would be waited for
+        long_ = {"P": len(prod) >= CO_LONG, "L": len(loss) >= CO_LONG}
+
+        def alternate(name):
+            turn[name] = turn.get(name, -1) + 1
+            return f"{name}{turn[name] & 1 if long_[name] else 0}"
+
+        def is_fresh(t):
+            return any(y[1] in fresh for y in t[2])
+
+        def split(terms):
+            """({species of prev: terms without it}, [(factor, terms without it)], single terms)"""
+            mine, many, single = {}, [], []
+            for c, op, ys in terms:
+                f = [y for y in ys if y[0] == "yn" and y[1] in prev]
+                assert len(f) <= 1
+                if f:
+                    ys = list(ys)
+                    ys.remove(f[0])
+                    mine.setdefault(f[0][1], []).append((c, op, ys))
+                else:
+                    (many if len(ys) >= 2 else single).append((c, op, ys))
+            groups = []
+            while many:
+                cnt: dict = {}
+                for _, _, ys in many:
+                    for v in set(ys):
+                        cnt[v] = cnt.get(v, 0) + 1
+                # a fresh factor first: what it multiplies can be summed before it arrives
+                f = max(cnt, key=lambda v: (v[1] in fresh, cnt[v], v[0], -v[1]))
+                if cnt[f] < 2 and f[1] not in fresh:
+                    break
+                g = []
+                for t in [t for t in many if f in t[2]]:
+                    many.remove(t)
+                    ys = list(t[2])
+                    ys.remove(f)
+                    g.append((t[0], t[1], ys))
+                groups.append((f, g))
+            return mine, groups, single + many
+
+        pm, pg, ps = split(prod)
+        lm, lg, ls = split(loss)
+        have = {}
+        waiting = sorted([("L", t) for t in ls] + [(f"H{i}", t) for i, k in enumerate(sorted(lm)) for t in lm[k]],
+                         key=lambda q: self.key(q[1]))
+
+        def put(q):
+            waiting.remove(q)
+            add(post if is_fresh(q[1]) else pre, alternate(q[0]) if q[0] == "L" else q[0], self.product(*q[1]))
+
+        def loss_of(pair):
+            for q in [q for q in waiting if _pair(q[1]) == pair and not is_fresh(q[1])]:
+                put(q)
+
+        def inner(g, name):
+            """A group's sum as an expression: two accumulators where it is long; (expression, fresh or not)"""
+            ways = 2 if len(g) >= CO_LONG else 1
+            var = [name + "ab"[w] for w in range(ways)]
+            number[0] += 1
+            me = number[0]
+            now = [t for t in sorted(g, key=self.key) if not is_fresh(t)]
+            later = [t for t in sorted(g, key=self.key) if is_fresh(t)]
+            for i, t in enumerate(now + later):
+                add(pre if i < len(now) else post, var[i % ways], self.product(*t), me)
+                loss_of(_pair(t))
+            return var[0] if ways == 1 else f"CO_ADD({var[0]}, {var[1]})", bool(later)
+
+        for i, k in enumerate(sorted(pm)):
+            have[(b, "P", k)] = inner(pm[k], f"G{i}")[0]
+        n = 0
+        for sums_, groups in (("P", pg), ("L", lg)):
+            for f, g in groups:
+                late = f[1] in fresh
+                e, deep = inner(g, f"{'ef'[sums_ == 'L']}{f[1]}" if late else f"g{n % 3}")
+                assert not deep or late
+                n += not late
+                add(post if late else pre, alternate(sums_), (self.y(f), e))
+        for t in sorted(ps, key=self.key):
+            add(post if is_fresh(t) else pre, alternate("P"), self.product(*t))
+            loss_of(_pair(t))
+        for q in list(waiting):
+            put(q)
+        for i, k in enumerate(sorted(lm)):
+            have[(b, "L", k)] = f"H{i}"
+        started: set[tuple] = set()
+
+        def text(st):
+            out = []
+            for var, sum_, (x, y) in st:
+                if (var, sum_) in started:
+                    out.append(f"{var} = CO_ADD({var}, {x});" if y is None else f"{var} = CO_FMA({x}, {y}, {var});")
+                else:
+                    out.append(f"{var} = {x};" if y is None else f"{var} = CO_MUL({x}, {y});")
+                started.add((var, sum_))
+            return out
+        pre, post = text(pre), text(post)
+        for nm in "PL":
+            v = [x for x in (nm + "0", nm + "1") if (x, 0) in started]
+            if v:
+                have[(b, nm, None)] = _added(v)
+        return pre, post, have
+
+
+def _segments(body, mine):
+    """The statements in segments of at most CO_SEG row pairs in tensor memory."""
+    import re
+    tok = re.compile(r"@(\d+)@")
+    segs, cur, rows = [], [], []
+    for st in body:
+        need = list(dict.fromkeys(int(x) // 2 for x in tok.findall(st) if int(x) // 2 in mine))
+        new = [r for r in need if r not in rows]
+        if cur and len(rows) + len(new) > CO_SEG:
+            segs.append((cur, rows))
+            cur, rows, new = [], [], need
+        cur.append(st)
+        rows = rows + new
+    return segs + [(cur, rows)]
+
+
+def _place(segs, mine):
+    """Tensor-memory columns of a warp's pairs: pairs that are loaded in the same segments side by side (in
+    twos, and the twos in twos), heaviest first, so that one wide load brings them."""
+    groups = [(p,) for p in sorted(mine)]
+    for _ in range(2):
+        at = {p: i for i, g in enumerate(groups) for p in g}
+        weight: dict = {}
+        for _, rows in segs:
+            have = sorted({at[p] for p in rows if all(q in rows for q in groups[at[p]])})
+            for i, x in enumerate(have):
+                for y in have[i + 1:]:
+                    weight[(x, y)] = weight.get((x, y), 0) + 1
+        taken, merged = set(), []
+        for (x, y), _w in sorted(weight.items(), key=lambda q: (-q[1], q[0])):
+            if x not in taken and y not in taken and len(groups[x]) == len(groups[y]):
+                taken |= {x, y}
+                merged.append(groups[x] + groups[y])
+        left = [g for i, g in enumerate(groups) if i not in taken]
+        full = max(len(g) for g in groups)
+        ones = [g for g in left if len(g) < full]
+        left = [g for g in left if len(g) == full]
+        while len(left) > 1:
+            merged.append(left.pop(0) + left.pop(0))
+        groups = merged + left + ones
+    return {p: 4 * i for i, p in enumerate(p for g in sorted(groups, key=len, reverse=True) for p in g)}
+
+
+def _bind(body, slots):
+    """Bind the row pairs of a warp's statements: those in `slots` (pair -> tensor-memory column) through two
+    register banks, loaded one segment ahead, the others from shared memory. Returns (statements, segments,
+    tensor-memory loads, shared-memory loads)."""
+    import re
+    tok = re.compile(r"@(\d+)@")
+    segs = _segments(body, slots)
+    out, live, name, nlds, ns, ntm = [], {}, {}, 0, 0, 0
+    places = []
+    for _, rows in segs:
+        # aligned neighbours in one load: four pairs, two pairs, one
+        cols = {slots[r]: r for r in rows}
+        order, lds = [], []
+        for n in (4, 2, 1):
+            for c in sorted(cols):
+                if c in cols and c % (4 * n) == 0 and all(c + 4 * i in cols for i in range(n)):
+                    lds.append((n, len(order), c, [cols[c + 4 * i] for i in range(n)]))
+                    order += [cols.pop(c + 4 * i) for i in range(n)]
+        places.append((order, lds))
+
+    def loads(si):
+        nonlocal ntm
+        ntm += len(places[si][1])
+        return [f"TM_LD{2 * n}({si % 2}, {q}, {c}, {', '.join(map(str, ps))});" for n, q, c, ps in places[si][1]]
+    def wait(si):
+        n = len(segs[si][1])
+        return [f"TM_WAIT({si % 2}, {n});"] if n else []
+    out += loads(0) + wait(0)
+    for si, (stmts, rows) in enumerate(segs):
+        slot = {r: q for q, r in enumerate(places[si][0])}
+        if si + 1 < len(segs):
+            out += loads(si + 1)
+        for st in stmts:
+            ns += 1
+            for x in tok.findall(st):
+                pr = int(x) // 2
+                if pr in slots:
+                    continue
+                if pr not in live or ns - live[pr] > CO_REUSE:
+                    name[pr] = f"s{nlds}"
+                    out.append(f"const double2 s{nlds} = RCS2({pr - CO_NT // 2});")
+                    nlds += 1
+                live[pr] = ns
+
+            def bind(m):
+                r = int(m.group(1))
+                if r // 2 in slots:
+                    return f"RCT({si % 2}, {2 * slot[r // 2] + r % 2})"
+                return f"{name[r // 2]}.{'xy'[r % 2]}"
+            out.append(tok.sub(bind, st))
+        if si + 1 < len(segs):
+            out += wait(si + 1)
+    return out, len(segs), ntm, nlds
+
+
+def gen_co_program(blocks) -> str:
+    """The species update with three warps per tile: two form the sums of the species, each from the terms
+    of its own row pairs, and the third closes them. The sums are grouped: terms that share a mass fraction
+    are added before they are multiplied by it, so that a term costs one fused multiply-add. Species that do
+    not enter one another's sums are closed together, in runs. While the closing warp forms a run, the others
+    already sum the next one: what a species of the run multiplies there is summed apart and waits for it in
+    one multiply-add. Terms, factors and the order of the species are those of the in-place program; only the
+    order of the additions and multiplications within a sum differs."""
+    import re
+    full = _grouped_sums(blocks)
+    assert [b["species"] for b in blocks] == list(range(LSP - 1))
+    assert all(not any(s) for s in full[CO_LAST + 1:]) and all(b["prod"] is None for b in blocks[CO_LAST + 1:])
+    assert len(full[CO_LAST][0]) == len(blocks[CO_LAST]["prod"])      # no extra terms in the sum they reuse
+    # the few soot-source terms are the closing warp's
+    sour = [[[t for t in side if t[1] is not None and t[1][0] == "SOUR"] for side in s] for s in full]
+    sums = [[[t for t in side if t[1] is not None and t[1][0] == "RC"] for side in s] for s in full]
+    assert all(len(a) + len(c) == len(d) for x, y, z in zip(sums, sour, full) for a, c, d in zip(x, y, z))
+    runs = _runs(sums)
+    nr = len(runs)
+    owner, share = _share_out(sums, runs)
+    macros, stats = [], []
+    flops = 19                                         # the two soot scalars
+
+    def operations(stmts):
+        return sum(st.count(" * ") + st.count(" + ") + st.count(" - ") + 2 * st.count("CO_FMA(") + st.count("CO_ADD(") +
+                   st.count("CO_MUL(") + st.count("CO_QUOT(") for st in stmts)
+
+    shadow_max = 1
+    handed = [[None] * CO_SUMS for _ in range(nr)]           # per run and warp: values in the order of its slots
+    slots_of = [0, 0]                                  # pair rows of each set of exchange buffers
+    base = [[0] * CO_SUMS for _ in range(nr)]
+
+    def program(w, place):
+        """Statements of summing warp w; place: tensor-memory columns of its pairs."""
+        em = _COEmit(place)
+        body: list[str] = []
+
+        def take(r, now):
+            return [f"CO_WAIT_Y({r & 1});"] + [f"CO_GET({3 * (r & 1) + i}, {k}, {int(k % CO_SUMS == w)}, {now});"
+                                             for i, k in enumerate(runs[r])]
+
+        def run_sums(r, before_post):
+            """The partial sums of run r; before_post: statements that bring the fresh values."""
+            prev = set(runs[r - 1]) if r > 0 else set()
+            fresh = set(runs[r - 2]) if r > 1 else set(runs[nr - 1]) if r == 0 else set()
+            st, vals, waited = [], {}, False
+            for b in runs[r]:
+                mine = [[t for t in side if share[r][_pair(t)] == w] for side in sums[b]]
+                pre, post, hv = em.sums(b, mine[0], mine[1], prev, fresh if not waited else set())
+                st += pre
+                if not waited:
+                    st += before_post
+                    waited = True
+                st += post
+                # the value's own variable, since the next species of the run uses the accumulators again
+                for key, e in hv.items():
+                    v = f"v{len(vals)}"
+                    st.append(f"{v} = {e};")
+                    vals[key] = v
+            keys = [k for k in _values(sums, runs[r], prev) if k in vals]
+            handed[r][w] = keys
+            for i in range(0, len(keys), 2):
+                st.append(f"CO_PUT(@@{r},{w},{i // 2}@@, {vals[keys[i]]}, {vals[keys[i + 1]] if i + 1 < len(keys) else '0.0'});")
+            return st + [f"CO_ARRIVE_P({r & 1});"]
+
+        # (the species of the last run are known from the pass before)
+        body += run_sums(0, take(nr - 1, 0))
+        body.append("CO_CHECK();")
+        for r in range(1, nr):
+            em.updated |= set(runs[r - 1])             # being closed now: an old value is the copy
+            body += run_sums(r, take(r - 2, 1) if r > 1 else [])
+        body += take(nr - 2, 1)
+        first = next(i for i, x in enumerate(body) if x == "CO_CHECK();")
+        body[first:first] = [f"YOS({m}) = YO({k});" for m, k in enumerate(em.shadow)]
+        return body, len(em.shadow)
+    bodies, places = [], []
+    for w in range(CO_SUMS):
+        mine = {p for p, v in enumerate(owner) if v == w}
+        place = {p: 4 * i for i, p in enumerate(sorted(mine))}
+        for _ in range(3):                             # places from the segments, statements in the places' order
+            body, n = program(w, place)
+            place = _place(_segments(body, mine), mine)
+        body, n = program(w, place)
+        shadow_max = max(shadow_max, n)
+        bodies.append(body)
+        places.append(place)
+    for r in range(nr):
+        n = 0
+        for w in range(CO_SUMS):
+            base[r][w] = n
+            n += (len(handed[r][w]) + 1) // 2
+        slots_of[r & 1] = max(slots_of[r & 1], n)
+
+    def slot(m):
+        r, w, i = (int(x) for x in m.group(1).split(","))
+        return str((slots_of[0] if r & 1 else 0) + base[r][w] + i)
+    mark = re.compile(r"@@(\d+,\d+,\d+)@@")
+    for w in range(CO_SUMS):
+        body = [mark.sub(slot, st) for st in bodies[w]]
+        flops += operations(body)
+        out, nseg, nt, ns = _bind(body, places[w])
+        stats.append((nseg, nt, ns, operations(body)))
+        names = sorted({m for st in body for m in re.findall(r"\b([PLvGHgef]\d+[ab]?)\b", st)})
+        macros.append(["#define UC_CO_SUMS_%d() do { \\" % w, f"    double {', '.join(names)}; \\"] +
+                      ["    " + x + " \\" for x in out] + ["} while (0)"])
+    # ---- the closing warp
+    close: list[str] = []
+    names = {"rest"}
+
+    def fetch(r):
+        """The partial sums of run r, added up over the warps."""
+        st, parts = [f"CO_WAIT_P({r & 1});"], {}
+        for w in range(CO_SUMS):
+            keys = handed[r][w]
+            for i in range(0, len(keys), 2):
+                x, y = f"x{w}{i // 2}", f"y{w}{i // 2}"
+                names.update((x, y))
+                st.append(f"CO_TAKE({(slots_of[0] if r & 1 else 0) + base[r][w] + i // 2}, {x}, {y});")
+                parts.setdefault(keys[i], []).append(x)
+                if i + 1 < len(keys):
+                    parts.setdefault(keys[i + 1], []).append(y)
+        total = {}
+        for j, (key, vs) in enumerate(sorted(parts.items(), key=lambda q: str(q[0]))):
+            v = f"t{r & 1}{j}"
+            names.add(v)
+            st.append(f"{v} = {_added(vs)};")
+            total[key] = v
+        return st, total
+
+    def faces(r):
+        return [f"CO_PF({k % window}, {k});" for k in (runs[r] if r < nr else range(CO_LAST + 1, LSP - 1) if r == nr else [])]
+    spans = [len(x) for x in runs] + [2]
+    window = max(sum(spans[i:i + 3]) for i in range(len(spans)))
+
+    def finish(k):
+        return [f"fnew = CO_FMA(sor2, YO({k}), q{k % 3});", f"rsd += fabs(YO({k}) - fnew);", f"CO_TAIL({k});"]
+    close += faces(0) + faces(1)
+    st, total = fetch(0)
+    close += st + ["CO_CHECK();"]
+    for r, run in enumerate(runs):
+        close += faces(r + 2)
+        for k in run:
+            e = {}
+            for side, nm in enumerate("PL"):
+                x = total.get((k, nm, None), "")
+                more = [(f"YO({key[2]})", v) for key, v in sorted(total.items(), key=lambda q: str(q[0]))
+                        if key[0] == k and key[1] == nm and key[2] is not None]
+                for c, op, ys in sour[k][side]:
+                    assert all(y[0] == "yn" or y[1] >= k for y in ys) and len(ys) <= 1
+                    more.append((f"SOUR({op[1]})" if c == 1.0 else f"({c!r} * SOUR({op[1]}))", f"YO({ys[0][1]})" if ys else None))
+                for f, v in more:
+                    if v is None:
+                        x = f"CO_ADD({x}, {f})" if x else f
+                    else:
+                        x = f"CO_FMA({f}, {v}, {x})" if x else f"CO_MUL({f}, {v})"
+                e[nm] = x
+            if k == CO_LAST:
+                close.append(f"rest = {e['P']};")      # argon and helium reuse the last production sum
+                e["P"] = "rest"
+            num = f"CO_FMA(DTW({k}), {e['P']}, RY0({k}))" if e["P"] else f"RY0({k})"
+            den = f"rho - FSS({k % window})"
+            close.append(f"n{k % 3} = ({num} - FNS({k % window})) * sor1;")
+            close.append(f"d{k % 3} = " + (f"CO_FMA(DTW({k}), {e['L']}, {den});" if e["L"] else f"{den};"))
+        # the next run's partial sums are fetched while the quotients are on their way
+        st, total = fetch(r + 1) if r + 1 < nr else ([], {})
+        close += [f"q{k % 3} = CO_QUOT(n{k % 3}, d{k % 3});" for k in run] + st
+        for i, k in enumerate(run):
+            close += finish(k) + [f"CO_GIVE({3 * (r & 1) + i}, {k});"]
+        close.append(f"CO_ARRIVE_Y({r & 1});")
+    for k in range(CO_LAST + 1, LSP - 1):
+        close.append(f"n{k % 3} = (CO_FMA(DTW({k}), rest, RY0({k})) - FNS({k % window})) * sor1;")
+        close.append(f"d{k % 3} = rho - FSS({k % window});")
+        close.append(f"q{k % 3} = CO_QUOT(n{k % 3}, d{k % 3});")
+        close += finish(k)
+    flops += operations(close)
+    macros.append(["#define UC_CO_CLOSE() do { \\", f"    double n0, n1, n2, d0, d1, d2, q0, q1, q2, fnew, {', '.join(sorted(names))}; \\"] +
+                  ["    " + x + " \\" for x in close] + ["} while (0)"])
+    # in the order of staging: (pair, column)
+    rows = [[(p, places[w][p]) for p in sorted(places[w])] for w in range(CO_SUMS)]
+    L = ["// Generated by unicorn_b200/mech/codegen.py: the species update (src/lib/solvesp.f:85-2806) with three",
+         "// warps per 32-cell tile. UC_CO_SUMS_0 and _1 are a pass of the two summing warps, UC_CO_CLOSE one of the",
+         f"// closing warp. RC slots 0..{CO_NT - 1} lie in tensor memory, each pair of slots (2p, 2p + 1) with the one",
+         "// summing warp that uses it (uc_co_pairs_w: the pairs in row order; uc_co_cols_w: the first of the four",
+         "// 32-bit columns of each); the others lie in shared memory as rows of pairs, RCS2(i). Accessors: TM_LD2(bank,",
+         "// q, col, p) loads pair p (column col) into slots 2q, 2q + 1 of a register bank, TM_LD4 and TM_LD8 two and four",
+         "// pairs in neighbouring columns, TM_WAIT(bank, n) waits for the loads of its n pairs, RCT(bank, i); CO_PUT",
+         "// (slot, a, b) publishes two partial sums, CO_TAKE(slot, a, b) reads them; CO_GIVE(buf, k) publishes the",
+         "// new Y of species k, CO_GET(buf, k, mine, now) takes it into YO(k) (mine: this warp also stores it; now: of",
+         "// this pass, else of the pass before). Even and odd runs use sets 0 and 1 of the buffers and barriers:",
+         "// CO_ARRIVE_P(set) by the summing warps, CO_WAIT_P(set) by the closing one, CO_ARRIVE_Y, CO_WAIT_Y the other way;",
+         "// CO_CHECK() may leave the program (no more passes). CO_PF(slot, k) fetches the face terms of species k",
+         "// (FSS, FNS); RY0(k) is rho times the old level's Y; DTW(k) is dt * WM(k); CO_QUOT(n, d) is the quotient;",
+         "// CO_FMA(a, b, c) = a * b + c, CO_MUL and CO_ADD are rounded as they stand, so that every kernel that runs the",
+         "// program computes a cell bit for bit the same.",
+         f"// {nr} runs: {' '.join('-'.join(map(str, sorted({x[0], x[-1]}))) for x in runs)}",
+         "// Per summing warp: " + "; ".join(f"{a} segments, {b} tensor-memory loads, {c} shared-memory pair loads, {d} "
+                                          "operations" for a, b, c, d in stats) + ".",
+         "#pragma once",
+         f"#define UC_CO_NT {CO_NT}", f"#define UC_CO_NS {LRX - CO_NT}", f"#define UC_CO_PIECE {CO_PIECE}",
+         f"#define UC_CO_SEG {CO_SEG}", f"#define UC_CO_SUMS {CO_SUMS}", f"#define UC_CO_NSHADOW {shadow_max}", f"#define UC_CO_LAST {CO_LAST}",
+         f"#define UC_CO_SLOTS {sum(slots_of)}", f"#define UC_CO_WINDOW {window}",
+         "// the last run: its species' buffers hold their values when a pass begins, handed over through the set",
+         f"#define UC_CO_LAST_SET {(nr - 1) & 1}", "#define UC_CO_LAST_RUN() do { " +
+         " ".join(f"CO_LAST_SPECIES({3 * ((nr - 1) & 1) + i}, {k});" for i, k in enumerate(runs[-1])) + " } while (0)",
+         "// operations per cell and pass (a multiply-add is two, a quotient one), the exchange between the warps included",
+         f"#define UC_UPDATE_FLOPS_PER_CELL_PASS {flops}"]
+    for w in range(CO_SUMS):
+        L.append(f"#define UC_CO_PAIRS_{w} {CO_PAIRS[w]}")
+    for m in macros:
+        L += m
+    for kind, guard in (("static __constant__ int16_t", "#ifdef __CUDACC__"), ("static const short", "#else")):
+        L.append(guard)
+        for w in range(CO_SUMS):
+            for i, nm in enumerate(("pairs", "cols")):
+                L.append(f"{kind} uc_co_{nm}_{w}[{len(rows[w])}] = {{{', '.join(str(x[i]) for x in rows[w])}}};")
+    L.append("#endif")
+    return "\n".join(L) + "\n"
+
+
 # ------------------------------------------------------------------ tables
 
 def fmt(v: float) -> str:
@@ -570,6 +1208,7 @@ def main():
                     if leaf.kind == "RC":
                         uses[leaf.idx] = uses.get(leaf.idx, 0) + 1
     (GEN / "update_program_tr.cuh").write_text(gen_tr_program(blocks, uses, gen_inplace_program.shadow))
+    (GEN / "update_program_co.cuh").write_text(gen_co_program(blocks))
     print(f"wrote {GEN / 'mech_tables.h'}, {GEN / 'update_program.cuh'} and {GEN / 'update_program_tr.cuh'}")
 
 
