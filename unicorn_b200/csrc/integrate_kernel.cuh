@@ -133,7 +133,7 @@ struct IntArgs {
 };
 
 constexpr size_t INT_SMEM =
-    PAIRTAB_BYTES + sizeof(double) * (size_t)(LRX * TILE + 3 * LSP * TILE + SC_N * TILE + 6 * TILE) + 64;
+    PAIRTAB_BYTES + sizeof(double) * (size_t)(LRX * TILE + 4 * LSP * TILE + SC_N * TILE + 6 * TILE + CHEM_POLY) + 64;
 static_assert(INT_SMEM <= 232448, "integrator tile does not fit in shared memory");
 
 // Total enthalpy of a cell at its own temperature, in the units of ENTH in
@@ -464,11 +464,12 @@ struct IntTile {
 };
 // the kernel's dynamic shared memory, laid out in this order
 constexpr size_t INT_OFF_RC = PAIRTAB_BYTES, INT_OFF_Y = INT_OFF_RC + sizeof(double) * LRX * TILE,
-                 INT_OFF_G = INT_OFF_Y + sizeof(double) * LSP * TILE, INT_OFF_Y0 = INT_OFF_G + sizeof(double) * LSP * TILE,
+                 INT_OFF_G = INT_OFF_Y + sizeof(double) * LSP * TILE, INT_OFF_Y0 = INT_OFF_G + sizeof(double) * 2 * LSP * TILE,
                  INT_OFF_C = INT_OFF_Y0 + sizeof(double) * LSP * TILE, INT_OFF_S = INT_OFF_C + sizeof(double) * SC_N * TILE,
-                 INT_OFF_BAR = INT_OFF_S + sizeof(double) * 6 * TILE, INT_OFF_QUIT = INT_OFF_BAR + 8;
+                 INT_OFF_POLY = INT_OFF_S + sizeof(double) * 6 * TILE,
+                 INT_OFF_BAR = INT_OFF_POLY + sizeof(double) * CHEM_POLY, INT_OFF_QUIT = INT_OFF_BAR + 8;
 static_assert(INT_OFF_QUIT + 8 <= INT_SMEM, "shared memory of the integrator");
-static_assert(2 * UC_CO_SLOTS <= LSP, "the partial sums take the place of the Gibbs functions");
+static_assert(UC_CO_SLOTS <= LSP, "the partial sums take the place of the Gibbs functions");
 // from the shared array itself, so that a function that is not inlined reads it with shared-memory loads
 __device__ __forceinline__ IntTile int_tile()
 {
@@ -598,6 +599,8 @@ __global__ void __launch_bounds__(NW * 32, 1) integrate_fp64_kernel(const IntArg
         mbar_wait_bounded(bar, 0, 1 << 20);
         return;
     }
+    double *sPoly = reinterpret_cast<double *>(smem + INT_OFF_POLY);  // [52][14]
+    for (int i = tid; i < CHEM_POLY; i += NW * 32) sPoly[i] = P.poly[i];
     const size_t np = a.npad;
     const double sor1 = a.sor1, sor2 = 1.0 - a.sor1;
 
@@ -635,20 +638,14 @@ __global__ void __launch_bounds__(NW * 32, 1) integrate_fp64_kernel(const IntArg
         __syncthreads();
         const int smax = s_smax;
         for (int st = 0; st < smax; ++st) {
-            if (warp == 0) {
-                const double TKD = tk * P.TSTR;
-                sC[SC_TK * TILE + lane] = tk;
-                sC[SC_TKD * TILE + lane] = TKD;
-                sC[SC_LNT * TILE + lane] = log(TKD);
-                sC[SC_RUT * TILE + lane] = (double)82.06f * TKD;
-                sC[SC_RHO * TILE + lane] = rho;
-                sC[SC_DMOLEA * TILE + lane] = rho * P.RSTR / P.WMSTR * 1.0e-06;
-                sC[SC_STMF * TILE + lane] = s1;
-                sC[SC_STND * TILE + lane] = s2;
-            }
+            if (warp == 0) tile_scalars(P, sC, lane, tk, rho, s1, s2);
             __syncthreads();
             if (!MIXED || tile_rates_mixed<NW>(P, a.tabm, sRC, sY, sYN, sC, sS, TILE, lane, lane, warp))
-                tile_rates_fp64<NW>(P, sTab, sRC, sY, sYN, sC, sS, TILE, lane, lane, warp);
+                tile_rates_fp64<NW>(P, sTab, sPoly, sY, sYN, sC, sS, TILE, lane, lane, warp, false,
+                                    [&](int p, double rc0, double rc1) {
+                                        sRC[(2 * p) * TILE + lane] = rc0;
+                                        sRC[(2 * p + 1) * TILE + lane] = rc1;
+                                    });
             __syncthreads();
             if (warp == 1) { while (int_sums<0>()) {} }
             else if (warp == 2) { while (int_sums<1>()) {} }

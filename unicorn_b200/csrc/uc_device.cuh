@@ -23,21 +23,38 @@ constexpr int ST_BAD_ORDER = 3;
 constexpr int ST_MMA_TIMEOUT = 4;
 constexpr int ST_RELAX_TIMEOUT = 5;
 
-// One reaction pair of the mechanism: forward slot 2p and reverse slot 2p+1
-// (0-based). Staged into shared memory by a bulk (TMA) copy at kernel start.
-struct __align__(16) PairTab {
+// One reaction pair of the mechanism as the reference's sources give it: forward slot 2p and reverse slot
+// 2p + 1 (0-based). Host side: the device tables are made from it.
+struct PairSrc {
     double akf, alf, exaf, akf_r;          // Arrhenius of the forward slot; AKF of the reverse slot
-    double aklow, allow, ealow, pad0;      // fall-off low-pressure limit (aklow = 0: none)
+    double aklow, allow, ealow;            // fall-off low-pressure limit (aklow = 0: none)
     double troe[4];                        // TROE(IR,1..4)
     int8_t has_rev, rut, qlen, dmole;      // reverse formula present; RUT power; q length; TB group of DMOLE
     int8_t rc_order0, rc_order1, rc_tb0, rc_tb1;   // RC assembly (order 0 = slot never written)
-    int8_t rc_len0, rc_len1, pad1[6];
+    int8_t rc_len0, rc_len1;
     int8_t qsp[8], qdiv[8];                // q = G[qsp0] (*|/) G[qsp1] ...
     int8_t rc_kind0[4], rc_idx0[4];        // post factors: kind 1 = *Y[idx], 0 = /WM[idx]
     int8_t rc_kind1[4], rc_idx1[4];
 };
-static_assert(sizeof(PairTab) == 144, "PairTab layout");
-constexpr int PAIRTAB_BYTES = NPAIR * (int)sizeof(PairTab);
+
+// The pair as the FP64 rate kernels evaluate it: k_f = akf T^alf exp(-exaf / T); k_r = k_f * (RUT power) * 1/q
+// with 1/q a product of rows of the table of G and 1/G; RC = c * rho^order * [third body] * k [* Y]. Rows name
+// scalar rows (SC_*, 0: none) of the tile, so nothing is decoded or divided per cell.
+struct __align__(16) PairTab {
+    double akf, alf, exaf, c0, c1, pad0;
+    uint8_t g[6], ng, rut;                 // rows of the G table (k: G_k, 52 + k: 1 / G_k); ng = 0: no reverse
+    uint8_t r0, t0, r1, t1;                // rows of rho^order (0: the slot is never written) and of the third body
+    uint8_t y0, y1, fall, pad1;            // species whose Y is a factor (255: none); 1 + fall-off entry (0: none)
+};
+static_assert(sizeof(PairTab) == 64, "PairTab layout");
+struct __align__(16) FallTab {
+    double aklow, allow, ealow, troe[4];
+    int dmole, pad;                        // scalar row of the third body
+};
+static_assert(sizeof(FallTab) == 64, "FallTab layout");
+constexpr int NFALL = 24;                  // entries of the fall-off table (the mechanism has 21)
+// both tables lie one after the other, staged into shared memory by bulk (TMA) copies at kernel start
+constexpr int PAIRTAB_BYTES = NPAIR * (int)sizeof(PairTab) + NFALL * (int)sizeof(FallTab);
 static_assert(PAIRTAB_BYTES % 16 == 0, "bulk copy size must be a multiple of 16 bytes");
 
 // Constants of one context: scales, tables prepared at set-up, and the
@@ -57,6 +74,8 @@ struct DevParams {
     // cp/R / W and h of every species as polynomials in T for Horner evaluation, per temperature range
     // (0: T <= TPOL1, 1: above): cp_k / W_k = sum_i cpc[i] T^i, h_k = T (sum_i hc[i] T^i) + hc[5]
     double cpc[LSP * 2 * 5], hc[LSP * 2 * 6];
+    // third bodies as weights of Y: row 0 TBODY (1 / W_k), rows 1..10 the groups
+    double tbw[11 * LSP];
     // third-body groups 1..10 (TBODY + sum sign*coef*Y/W)
     int16_t tb_off[11], tb_len[11];
     int8_t tb_sp[64], tb_sign[64], tb_hascoef[64];
@@ -73,7 +92,14 @@ struct DevParams {
     // reaction pairs assigned to each warp (balanced by cost)
     int16_t pair_of_warp[CHEM_WARPS][24];
     int8_t npair_of_warp[CHEM_WARPS];
+    int soot_warp;                        // the warp (of 16) that forms the soot sources
 };
+
+// Rounded as written (no contraction of a product into a neighbouring sum, which the compiler may do one way or
+// the other): for code that several kernels run and that has to give a cell the same bits in each.
+#define CO_FMA(a, b, c) __fma_rn(a, b, c)
+#define CO_MUL(a, b) __dmul_rn(a, b)
+#define CO_ADD(a, b) __dadd_rn(a, b)
 
 // ------------------------------------------------------------------ TMA / mbarrier
 

@@ -161,7 +161,7 @@ static int set_err(uc_ctx *c, int code, const char *fmt, ...)
 // Tables and scales of src/unicornd-mild-sd-5.f:327-483 (all reactions on,
 // IRSW=1), written for the device parameter block. Literal constants keep
 // the reference's single-precision kind where it has one.
-static void build_params(const uc_inputs &in, DevParams &P, std::vector<PairTab> &tab, std::vector<PairTabM> &tabm,
+static void build_params(const uc_inputs &in, DevParams &P, std::vector<uint8_t> &dev_tab, std::vector<PairTabM> &tabm,
                          uc_scales &sc)
 {
     const double RUCAL = F32(1.9872), GASC = F32(8.3144);
@@ -280,10 +280,10 @@ static void build_params(const uc_inputs &in, DevParams &P, std::vector<PairTab>
     memcpy(P.ra_sp, uc_ra_sp, sizeof(P.ra_sp));
 
     // reaction-pair table
-    tab.assign(NPAIR, PairTab{});
+    std::vector<PairSrc> tab(NPAIR, PairSrc{});
     std::vector<double> pcost(NPAIR);
     for (int p = 0; p < NPAIR; ++p) {
-        PairTab &T = tab[p];
+        PairSrc &T = tab[p];
         memset(&T, 0, sizeof(T));
         const int r0 = 2 * p, r1 = 2 * p + 1;
         T.akf = AKF[r0]; T.alf = ALF[r0]; T.exaf = EXAF[r0]; T.akf_r = AKF[r1];
@@ -301,7 +301,57 @@ static void build_params(const uc_inputs &in, DevParams &P, std::vector<PairTab>
             if (t < T.rc_len0) { T.rc_kind0[t] = uc_rc_kind[r0 * UC_PMAX + t]; T.rc_idx0[t] = uc_rc_idx[r0 * UC_PMAX + t]; }
             if (t < T.rc_len1) { T.rc_kind1[t] = uc_rc_kind[r1 * UC_PMAX + t]; T.rc_idx1[t] = uc_rc_idx[r1 * UC_PMAX + t]; }
         }
-        pcost[p] = 3.0 + (T.has_rev ? 1.0 + 0.5 * T.qlen : 0.0) + (T.aklow != 0.0 ? 6.0 : 0.0);
+        // instructions of the rate kernel, roughly: an exponential and the assembly, a reverse rate, and for a
+        // fall-off pair a low-pressure rate and the blend (up to four exponentials, two logarithms and a power)
+        pcost[p] = 6.0 + (T.has_rev ? 1.5 : 0.0) + (T.aklow != 0.0 ? (T.troe[1] == 0.0 || T.troe[0] == 0.0 ? 20.0 : 40.0) : 0.0);
+    }
+    // tables of the FP64 rate kernels
+    dev_tab.assign(PAIRTAB_BYTES, 0);
+    PairTab *pt = reinterpret_cast<PairTab *>(dev_tab.data());
+    FallTab *ft = reinterpret_cast<FallTab *>(dev_tab.data() + NPAIR * sizeof(PairTab));
+    const double CC[4] = {0.0, P.C1ST, P.C2ND, P.C3RD};
+    const uint8_t rho_row[4] = {0, SC_RHO, SC_RHO2, SC_RHO3};
+    for (int p = 0, nf = 0; p < NPAIR; ++p) {
+        const PairSrc &T = tab[p];
+        PairTab &D = pt[p];
+        D.akf = T.akf; D.alf = T.alf; D.exaf = T.exaf;
+        if (T.has_rev) {                   // (AKF of a reverse slot is 1)
+            std::vector<uint8_t> over, under;          // q = prod over / prod under; 1/q from them in turn, so
+            for (int t = 0; t < T.qlen; ++t)           // that the partial products stay near their size
+                (t > 0 && T.qdiv[t] ? under : over).push_back((uint8_t)T.qsp[t]);
+            for (size_t t = 0; t < std::max(over.size(), under.size()); ++t) {
+                if (t < over.size()) D.g[D.ng++] = (uint8_t)(LSP + over[t]);
+                if (t < under.size()) D.g[D.ng++] = under[t];
+            }
+            D.rut = T.rut < 0 ? SC_IRUT : T.rut > 0 ? SC_RUT : 0;
+        }
+        auto assemble = [&](int order, int tb, int len, const int8_t *kind, const int8_t *idx, double &c, uint8_t &r,
+                            uint8_t &t, uint8_t &y) {
+            c = CC[order];
+            r = rho_row[order];
+            t = tb >= 0 ? (uint8_t)(SC_TB0 + tb) : 0;
+            y = 255;
+            for (int i = 0; i < len; ++i)
+                if (kind[i]) y = (uint8_t)idx[i];
+                else c = c / P.WM[idx[i]];
+        };
+        assemble(T.rc_order0, T.rc_tb0, T.rc_len0, T.rc_kind0, T.rc_idx0, D.c0, D.r0, D.t0, D.y0);
+        assemble(T.rc_order1, T.rc_tb1, T.rc_len1, T.rc_kind1, T.rc_idx1, D.c1, D.r1, D.t1, D.y1);
+        if (T.aklow != 0.0 && nf < NFALL) {
+            FallTab &F = ft[nf];
+            F.aklow = T.aklow; F.allow = T.allow; F.ealow = T.ealow;
+            for (int c = 0; c < 4; ++c) F.troe[c] = T.troe[c];
+            F.dmole = SC_TB0 + T.dmole;
+            D.fall = (uint8_t)++nf;
+        }
+    }
+    for (int g = 0; g < 11; ++g) {
+        double *w = P.tbw + g * LSP;
+        for (int k = 0; k < LSP; ++k) w[k] = 1.0 / P.WM[k];
+        for (int t = 0; g > 0 && t < P.tb_len[g]; ++t) {
+            const int i = P.tb_off[g] + t, k = P.tb_sp[i];
+            w[k] += P.tb_sign[i] * (P.tb_hascoef[i] ? P.tb_coef[i] : 1.0) / P.WM[k];
+        }
     }
     // balance pairs and species over the warps (longest first onto the least loaded warp)
     auto balance = [](const std::vector<double> &cost, int nw, int cap, std::vector<std::vector<int>> &out) {
@@ -323,7 +373,7 @@ static void build_params(const uc_inputs &in, DevParams &P, std::vector<PairTab>
     tabm.assign(NPAIR, PairTabM{});
     const double CO[4] = {0.0, P.C1ST, P.C2ND, P.C3RD};
     for (int p = 0; p < NPAIR; ++p) {
-        const PairTab &T = tab[p];
+        const PairSrc &T = tab[p];
         PairTabM &M = tabm[p];
         memset(&M, 0, sizeof(M));
         M.lnakf = T.akf > 0.0 ? log(T.akf) : -1.0e300;
@@ -350,11 +400,13 @@ static void build_params(const uc_inputs &in, DevParams &P, std::vector<PairTab>
         M.lnc1 = l1 + (T.akf_r > 0.0 ? log(T.akf_r) : 0.0);
     }
     std::vector<std::vector<int>> pw, sw;
-    balance(pcost, CHEM_WARPS, 24, pw);
-    for (int w = 0; w < CHEM_WARPS; ++w) {
-        P.npair_of_warp[w] = (int8_t)pw[w].size();
-        for (size_t i = 0; i < pw[w].size(); ++i) P.pair_of_warp[w][i] = (int16_t)pw[w][i];
-    }
+    pcost.push_back(60.0);             // the soot sources, as one more item
+    balance(pcost, CHEM_WARPS, 25, pw);
+    for (int w = 0; w < CHEM_WARPS; ++w)
+        for (int p : pw[w]) {
+            if (p == NPAIR) P.soot_warp = w;
+            else if (P.npair_of_warp[w] < 24) P.pair_of_warp[w][P.npair_of_warp[w]++] = (int16_t)p;
+        }
     std::vector<double> scost(LSP);
     for (int k = 0; k < LSP; ++k) scost[k] = 8.0 + 2.0 * uc_prd_len[k] + 2.5 * uc_loss_len[k];
     balance(scost, CHEM_WARPS, MAX_SPEC_PER_WARP, sw);
@@ -569,7 +621,7 @@ extern "C" int uc_init(const uc_inputs *in, int ncell, int device, uc_ctx **out)
         ctx->npad = ctx->ntile * TILE;
         ctx->hP = new (std::nothrow) DevParams();
         if (!ctx->hP) { rc = UC_E_NOMEM; break; }
-        std::vector<PairTab> tab;
+        std::vector<uint8_t> tab;
         std::vector<PairTabM> tabm;
         build_params(*in, *ctx->hP, tab, tabm, ctx->sc);
         if (cudaMalloc((void **)&ctx->dP, sizeof(DevParams)) != cudaSuccess ||

@@ -147,9 +147,6 @@ __device__ __forceinline__ double co_quot(double n, double d)
     return m == m ? __fma_rn(m, r, q) : q0;
 }
 
-#define CO_FMA(a, b, c) __fma_rn(a, b, c)
-#define CO_MUL(a, b) __dmul_rn(a, b)
-#define CO_ADD(a, b) __dadd_rn(a, b)
 __device__ __forceinline__ void co_st2(double *p, double a, double b)
 {
     asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(smem_u32(p)), "d"(a), "d"(b));

@@ -762,12 +762,13 @@ def _place(segs, mine):
     return {p: 4 * i for i, p in enumerate(p for g in sorted(groups, key=len, reverse=True) for p in g)}
 
 
-def _bind(body, slots):
+def _bind(body, slots, first=None, shared="RCS2"):
     """Bind the row pairs of a warp's statements: those in `slots` (pair -> tensor-memory column) through two
     register banks, loaded one segment ahead, the others from shared memory. Returns (statements, segments,
     tensor-memory loads, shared-memory loads)."""
     import re
     tok = re.compile(r"@(\d+)@")
+    first = CO_NT // 2 if first is None else first     # row pair of the first shared-memory row
     segs = _segments(body, slots)
     out, live, name, nlds, ns, ntm = [], {}, {}, 0, 0, 0
     places = []
@@ -802,7 +803,7 @@ def _bind(body, slots):
                     continue
                 if pr not in live or ns - live[pr] > CO_REUSE:
                     name[pr] = f"s{nlds}"
-                    out.append(f"const double2 s{nlds} = RCS2({pr - CO_NT // 2});")
+                    out.append(f"const double2 s{nlds} = {shared}({pr - first});")
                     nlds += 1
                 live[pr] = ns
 
@@ -1036,6 +1037,62 @@ def gen_co_program(blocks) -> str:
     return "\n".join(L) + "\n"
 
 
+# ------------------------------------------------------------------ species source terms
+
+OM_WARPS = 16
+
+
+def gen_omega_program(mech: dict) -> str:
+    """The gain sum P_k and the loss sum L_k (the loss terms with one Y_k factored out, so that the production
+    is P_k - Y_k L_k and d(omega_k)/dY_k is -L_k) of every species from the PRD lists of
+    src/lib/solveh.f:677-1133, as straight-line code for the warps of a tile: each sum is one warp's, longest
+    first onto the least loaded. Terms that share a mass fraction are added before they are multiplied by it."""
+    import re
+    units = []
+    for key, terms in mech["prd"].items():
+        k = int(key) - 1
+        gain, loss = [], []
+        for s, fac in terms or []:
+            if fac[-1][0] == "SRA":
+                continue                               # SRA(i) = 0.0 (src/lib/solveh.f:671-676)
+            assert fac[-1][0] == "RA" and all(f[0] == "num" for f in fac[:-1])
+            r = fac[-1][1] - 1
+            if mech["ra"][str(r + 1)] is None:
+                continue                               # a slot that is never written: its RC is zero
+            ys = [("yo", x - 1) for x in mech["ra"][str(r + 1)]]
+            coef = 1.0
+            for f in fac[:-1]:
+                coef *= f[1]
+            if s > 0:
+                gain.append((coef, ("RC", r), ys))
+            else:
+                ys.remove(("yo", k))
+                loss.append((coef, ("RC", r), ys))
+        units += [(k, "P", gain), (k, "L", loss)]
+    load = [0.0] * OM_WARPS
+    mine: list[list] = [[] for _ in range(OM_WARPS)]
+    for u in sorted(units, key=lambda u: (-len(u[2]), u[0], u[1])):
+        w = min(range(OM_WARPS), key=lambda w: load[w])
+        mine[w].append(u)
+        load[w] += 2.0 + 1.6 * len(u[2])
+    tok = re.compile(r"@(\d+)@")
+    L = ["// Generated by unicorn_b200/mech/codegen.py: the species' gain and loss sums from the PRD lists of",
+         "// src/lib/solveh.f:677-1133, shared out over the warps of a tile: UC_OMEGA_w() is warp w's part.",
+         "// Requires RCP(p), the pair (RC(2p), RC(2p + 1)) of the cell as a double2, YO(k), and OM_PUT(k, v) and",
+         "// OM_PUT(52 + k, v), which store P_k and L_k; CO_FMA, CO_MUL, CO_ADD as in the species update.",
+         "#pragma once", f"#define UC_OM_WARPS {OM_WARPS}"]
+    for w, us in enumerate(mine):
+        em, body = _COEmit(), []
+        for k, nm, terms in us:
+            pre, post, have = em.sums(k, terms if nm == "P" else [], terms if nm == "L" else [], set(), set())
+            assert not post
+            body += pre + [f"OM_PUT({k + (LSP if nm == 'L' else 0)}, {have.get((k, nm, None), '0.0')});"]
+        out, _, _, _ = _bind(body, {}, 0, "RCP")
+        names = sorted({m for st in body for m in re.findall(r"\b([PLvGHgef]\d+[ab]?)\b", st)})
+        L += ["#define UC_OMEGA_%d() do { \\" % w, f"    double {', '.join(names)}; \\"] + ["    " + x + " \\" for x in out] + ["} while (0)"]
+    return "\n".join(L) + "\n"
+
+
 # ------------------------------------------------------------------ tables
 
 def fmt(v: float) -> str:
@@ -1209,6 +1266,7 @@ def main():
                         uses[leaf.idx] = uses.get(leaf.idx, 0) + 1
     (GEN / "update_program_tr.cuh").write_text(gen_tr_program(blocks, uses, gen_inplace_program.shadow))
     (GEN / "update_program_co.cuh").write_text(gen_co_program(blocks))
+    (GEN / "omega_program.cuh").write_text(gen_omega_program(mech))
     print(f"wrote {GEN / 'mech_tables.h'}, {GEN / 'update_program.cuh'} and {GEN / 'update_program_tr.cuh'}")
 
 
