@@ -2,7 +2,10 @@
 tile and one cell, one tile more than the GPU has SMs (the kernels' second round, whose inputs the rate kernel
 loads ahead) and one more than three per SM, against the oracle.
 
-Tolerances as in test_gpu_parity.py: RC and d(omega)/dY 1e-11 relative; QDSP 1e-11 of the gross rate; QDOT, a
+The properties at the edges of theirs (8 or 16 cells a block, by the field's size) and of the sub-mixture: more
+than 32 species in it, one species alone, N2 alone.
+
+Tolerances as in test_gpu_parity.py: mu, lambda, D_k, cp 1e-11 relative, h 1e-10; RC and d(omega)/dY 1e-11 relative; QDSP 1e-11 of the gross rate; QDOT, a
 sum of 52 products QDSP_k h_k, 1e-11 of the sum of the gross rates times |h_k|; Y after the update 1e-9."""
 import numpy as np
 import pytest
@@ -43,3 +46,30 @@ def test_rates_and_update_at_tile_edges(cuda, oracle, n):
     yo, _, po = oracle.species_update(rho, y, rc, sour, 1e-3, isor=2, tol=0.0)
     assert passes == po
     assert_rel(yg, yo, 1e-9, 1e-18, "Y after two passes")
+
+
+@pytest.mark.parametrize("n", [1, 7, 9, 32 * 148, 32 * 148 + 1, 512 * 148 + 17])
+def test_props_and_cp_h_at_tile_edges(cuda, oracle, n):
+    tk, rho, y = random_state(oracle, n, 60 + n % 7)
+    y = y.copy()
+    m = len(range(0, n, 5))
+    y[:, ::5] = np.random.default_rng(1).uniform(0.005, 0.03, (52, m))      # all 52 species in the sub-mixture
+    y[:, 1::7] = 1e-12                                                      # one species alone
+    y[12, 1::7] = 1.0 - 51e-12
+    y[:, 2::7] = 0.0                                                        # N2 alone
+    y[51, 2::7] = 1.0
+    y /= y.sum(0)
+    with cuda.UniChem(n) as u:
+        u.upload(tk, rho, y)
+        mu, lam, d = u.props()
+        cp, h = u.cp_h()
+        yc = u.download()[2]
+    yo, mu_o, lam_o, d_o, nsub = oracle.props(tk, y)
+    assert n < 6 or (nsub.max() > 32 and nsub.min() <= 2)
+    assert np.array_equal(yc, yo)
+    assert_rel(mu, mu_o, 1e-11, 0, "mu")
+    assert_rel(lam, lam_o, 1e-11, 0, "lambda")
+    assert_rel(d, d_o, 1e-11, 0, "D_k")
+    assert_rel(cp, oracle.cp(tk, yo), 1e-11, 0, "cp")
+    hm = oracle.enthalpy(tk, yo)[1]
+    assert_rel(h, hm, 1e-10, 1e-12 * np.abs(hm).max(), "h")

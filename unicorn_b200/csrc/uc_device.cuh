@@ -14,6 +14,7 @@ constexpr int TILE = 32;                 // cells per tile = lanes of a warp
 constexpr int CHEM_WARPS = 16;           // warps of the rate/omega kernel
 constexpr int CHEM_THREADS = CHEM_WARPS * 32;
 constexpr int MAX_SPEC_PER_WARP = 8;
+constexpr int PROP_ROWS = 24;            // see DevParams::prow
 
 // status words written by kernels (device side; the host maps them to UC_E*)
 constexpr int ST_OK = 0;
@@ -74,6 +75,12 @@ struct DevParams {
     // cp/R / W and h of every species as polynomials in T for Horner evaluation, per temperature range
     // (0: T <= TPOL1, 1: above): cp_k / W_k = sum_i cpc[i] T^i, h_k = T (sum_i hc[i] T^i) + hc[5]
     double cpc[LSP * 2 * 5], hc[LSP * 2 * 6];
+    // the FP64 property kernel's tables, species fastest (lane = species): per temperature range rows 0-4
+    // the Eucken factor's polynomial (0.115 + 0.354 cp/R), 5-10 cdia^2 times the Omega(2,2) fit, 11 CONVRC / W_kk,
+    // 12 CONVRM W_kk (W_kk = WMIK of the species with itself), 13-17 cpc, 18-23 hc; and for the pair
+    // (b, k) at b * LSP + k: 1 / WMCD, WMIK(k, b), 1 / DWMIK(k, b) (RETLJ1 is symmetric)
+    double prow[2][PROP_ROWS][LSP];
+    double piw[LSP * LSP], pw[LSP * LSP], pid[LSP * LSP];
     // third bodies as weights of Y: row 0 TBODY (1 / W_k), rows 1..10 the groups
     double tbw[11 * LSP];
     // third-body groups 1..10 (TBODY + sum sign*coef*Y/W)

@@ -263,6 +263,23 @@ static void build_params(const uc_inputs &in, DevParams &P, std::vector<uint8_t>
             P.ETLJ4[ij] = P.ETLJ3[ij] * P.ETLJ1[ij];
             P.RETLJ1[ij] = 1.0 / P.ETLJ1[ij];
         }
+    for (int r = 0; r < 2; ++r)         // the property kernel's tables
+        for (int k = 0; k < LSP; ++k) {
+            auto row = [&](int i) -> double & { return P.prow[r][i][k]; };
+            for (int i = 0; i < 5; ++i) row(i) = F32(0.354) * uc_poly[k * 14 + 7 * r + i];
+            row(0) += F32(0.115);
+            for (int i = 0; i < 6; ++i) row(5 + i) = uc_cdia[k] * uc_cdia[k] * uc_om22[k * 12 + 6 * r + i];
+            row(11) = P.CONVRC / P.WMIK[k * LSP + k];
+            row(12) = P.CONVRM * P.WMIK[k * LSP + k];
+            for (int i = 0; i < 5; ++i) row(13 + i) = P.cpc[(k * 2 + r) * 5 + i];
+            for (int i = 0; i < 6; ++i) row(18 + i) = P.hc[(k * 2 + r) * 6 + i];
+        }
+    for (int b = 0; b < LSP; ++b)
+        for (int k = 0; k < LSP; ++k) {
+            P.piw[b * LSP + k] = 1.0 / P.WMCD[k * LSP + b];
+            P.pw[b * LSP + k] = P.WMIK[k * LSP + b];
+            P.pid[b * LSP + k] = 1.0 / P.DWMIK[k * LSP + b];
+        }
     for (int g = 0; g < 11; ++g) { P.tb_off[g] = uc_tb_off[g]; P.tb_len[g] = uc_tb_len[g]; }
     const int ntb = (int)(sizeof(uc_tb_sp) / sizeof(uc_tb_sp[0]));
     for (int t = 0; t < ntb; ++t) {
@@ -993,13 +1010,14 @@ static int props_impl(uc_ctx *ctx, int precision, double *vmu, double *vtc, doub
     RET_IF(dalloc(ctx, &ctx->vtc, ctx->npad));
     RET_IF(dalloc(ctx, &ctx->vdf, (size_t)LSP * ctx->npad));
     PropArgs a{ctx->dP, ctx->tk, ctx->y, ctx->vmu, ctx->vtc, ctx->vdf, ctx->n, ctx->npad};
-    const int grid = std::min((ctx->n + 127) / 128, ctx->nsm * 16);
     int slot;
     prof_begin(ctx, UC_K_PROPS, slot);
     if (precision == UC_MIXED)
-        props_mixed_kernel<<<grid, 128, 0, ctx->stream>>>(a);
+        props_mixed_kernel<<<std::min((ctx->n + 127) / 128, ctx->nsm * 16), 128, 0, ctx->stream>>>(a);
+    else if (ctx->n > PROP_SMALL * ctx->nsm)
+        props_fp64_kernel<16><<<std::min((ctx->n + 15) / 16, ctx->nsm * 8), PROP_THREADS, 0, ctx->stream>>>(a);
     else
-        props_kernel<double><<<grid, 128, 0, ctx->stream>>>(a);
+        props_fp64_kernel<8><<<std::min((ctx->n + 7) / 8, ctx->nsm * 8), PROP_THREADS, 0, ctx->stream>>>(a);
     prof_end(ctx, slot);
     CK(cudaGetLastError());
     if (vmu || vtc || vdf) {
@@ -1024,13 +1042,15 @@ static int cp_h_impl(uc_ctx *ctx, int precision, double *cp, double *h)
     RET_IF(dalloc(ctx, &ctx->cp, ctx->npad));
     RET_IF(dalloc(ctx, &ctx->h, ctx->npad));
     CpHArgs a{ctx->dP, ctx->tk, ctx->y, ctx->cp, ctx->h, ctx->n, ctx->npad};
-    const int grid = std::min((ctx->n + 255) / 256, ctx->nsm * 8);
     int slot;
     prof_begin(ctx, UC_K_CPH, slot);
     // cp and h stay FP64 in the mixed form too: the kernel is bound by reading the 52 Y rows, and h is
     // a signed sum (formation enthalpies) that FP32 cannot hold to 1e-6 of itself
     (void)precision;
-    cp_h_kernel<double><<<grid, 256, 0, ctx->stream>>>(a);
+    if (ctx->n > CPH_SMALL * ctx->nsm)
+        cp_h_kernel<<<std::min((ctx->n + 255) / 256, ctx->nsm * 8), 256, 0, ctx->stream>>>(a);
+    else
+        cp_h_small_kernel<<<std::min((ctx->n + 31) / 32, ctx->nsm * 8), CPH_WARPS * 32, 0, ctx->stream>>>(a);
     prof_end(ctx, slot);
     CK(cudaGetLastError());
     if (cp || h) {
