@@ -22,6 +22,8 @@
 // closes them; the two forms of the integration thus compute a cell the same way) and
 // RC and Y in shared memory; the closure and the Newton for T run on warp 0 (lane = cell).
 #pragma once
+#include <cstddef>
+
 #include "chem_kernel.cuh"
 #include "chem_mixed_kernel.cuh"
 #include "update_tr_kernel.cuh"
@@ -136,24 +138,42 @@ constexpr size_t INT_SMEM =
     PAIRTAB_BYTES + sizeof(double) * (size_t)(LRX * TILE + 4 * LSP * TILE + SC_N * TILE + 6 * TILE + CHEM_POLY) + 64;
 static_assert(INT_SMEM <= 232448, "integrator tile does not fit in shared memory");
 
+// A1..A6 of solveh.f:1186-1205 for one temperature range: sums over the species of Y_k times tabulated coefficients
+// (a fused multiply-add each, where the reference's expression divides twice per term: with those divisions the
+// T Newton of 32,768 cells took 112 us, without them 22 us).
+__device__ __forceinline__ void newton_sums(const DevParams &P, int range, const double *y, int ys, double (&A)[6])
+{
+#pragma unroll
+    for (int i = 0; i < 6; ++i) A[i] = 0.0;
+#pragma unroll
+    for (int k = 0; k < LSP; ++k) {
+        const double2 *c = reinterpret_cast<const double2 *>(P.tco[range][k]);
+        const double yk = y[k * ys];
+        const double2 c0 = __ldg(c), c1 = __ldg(c + 1), c2 = __ldg(c + 2);
+        A[0] = CO_FMA(c0.x, yk, A[0]);
+        A[1] = CO_FMA(c0.y, yk, A[1]);
+        A[2] = CO_FMA(c1.x, yk, A[2]);
+        A[3] = CO_FMA(c1.y, yk, A[3]);
+        A[4] = CO_FMA(c2.x, yk, A[4]);
+        A[5] = CO_FMA(c2.y, yk, A[5]);
+    }
+}
+static_assert(offsetof(DevParams, tco) % 16 == 0, "the Newton's coefficients are read two at a time");
+
+// A1 T + A2 T^2 + ... + A6
+__device__ __forceinline__ double newton_h(const double (&A)[6], double T)
+{
+    return CO_FMA(CO_FMA(CO_FMA(CO_FMA(CO_FMA(A[4], T, A[3]), T, A[2]), T, A[1]), T, A[0]), T, A[5]);
+}
+
 // Total enthalpy of a cell at its own temperature, in the units of ENTH in
 // solveh.f:1186-1205; y has stride ys between species.
 __device__ __forceinline__ double enthalpy_total(const DevParams &P, double tk, const double *y, int ys)
 {
     const double TKD = tk * P.TSTR;
-    const int ip = TKD > UC_TPOL1 ? 7 : 0;
-    double A1 = 0.0, A2 = 0.0, A3 = 0.0, A4 = 0.0, A5 = 0.0, A6 = 0.0;
-    for (int k = 0; k < LSP; ++k) {
-        const double *a = P.poly + k * 14 + ip;
-        const double yk = y[k * ys];
-        A1 = A1 + a[0] * yk / P.WM[k];
-        A2 = A2 + a[1] * yk / P.WM[k] / 2.0;
-        A3 = A3 + a[2] * yk / P.WM[k] / 3.0;
-        A4 = A4 + a[3] * yk / P.WM[k] / 4.0;
-        A5 = A5 + a[4] * yk / P.WM[k] / 5.0;
-        A6 = A6 + a[5] * yk / P.WM[k];
-    }
-    return ((A1 + (A2 + (A3 + (A4 + A5 * TKD) * TKD) * TKD) * TKD) * TKD + A6) * P.GASC / P.WMSTR;
+    double A[6];
+    newton_sums(P, TKD > UC_TPOL1 ? 1 : 0, y, ys, A);
+    return newton_h(A, TKD) * P.GASC / P.WMSTR;
 }
 
 // Newton for T at total enthalpy ENTH (solveh.f:1186-1234). Returns tk;
@@ -162,42 +182,42 @@ __device__ __forceinline__ double enthalpy_total(const DevParams &P, double tk, 
 __device__ __forceinline__ double temperature_at(const DevParams &P, double tk, const double *y, int ys, double ENTH,
                                                  bool *conv)
 {
-    int IPL = 0;
     double TPOLY = UC_TPOL1;
     double TKD = tk * P.TSTR;
-    double A1, A2, A3, A4, A5, A6;
-    for (int guard = 0; guard < 3; ++guard) {
+    double A[6];
+#pragma unroll 1
+    for (int range = 0;; range = 1) {
         if (TKD > TPOLY) TKD = TPOLY / 2.0;
-        A1 = A2 = A3 = A4 = A5 = A6 = 0.0;
-        for (int k = 0; k < LSP; ++k) {
-            const double *p = P.poly + k * 14 + IPL;
-            const double yk = y[k * ys];
-            A1 = A1 + p[0] * yk / P.WM[k];
-            A2 = A2 + p[1] * yk / P.WM[k] / 2.0;
-            A3 = A3 + p[2] * yk / P.WM[k] / 3.0;
-            A4 = A4 + p[3] * yk / P.WM[k] / 4.0;
-            A5 = A5 + p[4] * yk / P.WM[k] / 5.0;
-            A6 = A6 + p[5] * yk / P.WM[k];
-        }
-        const double FUNT =
-            ((A1 + (A2 + (A3 + (A4 + A5 * TPOLY) * TPOLY) * TPOLY) * TPOLY) * TPOLY + A6) * P.GASC / P.WMSTR - ENTH;
-        if (FUNT >= 1.0e-07) break;
-        if (IPL >= 7) break;
-        IPL = 7;
+        newton_sums(P, range, y, ys, A);
+        const double FUNT = newton_h(A, TPOLY) * P.GASC / P.WMSTR - ENTH;
+        if (FUNT >= 1.0e-07 || range == 1) break;
         if (TKD <= TPOLY) TKD = UC_TPOL2 / 2.0;
         TPOLY = UC_TPOL2;
     }
+    const double h0 = ENTH * P.WMSTR / P.GASC;
     *conv = false;
+#pragma unroll 1
     for (int it = 1; it <= 100; ++it) {
-        const double num = __fma_rn(__fma_rn(__fma_rn(__fma_rn(__fma_rn(A5, TKD, A4), TKD, A3), TKD, A2), TKD, A1), TKD, A6);
-        const double den = __fma_rn(__fma_rn(__fma_rn(__fma_rn(5.0 * A5, TKD, 4.0 * A4), TKD, 3.0 * A3), TKD, 2.0 * A2), TKD, A1);
-        const double DTKD = (num - ENTH * P.WMSTR / P.GASC) / den;
+        const double den = CO_FMA(CO_FMA(CO_FMA(CO_FMA(5.0 * A[4], TKD, 4.0 * A[3]), TKD, 3.0 * A[2]), TKD, 2.0 * A[1]), TKD, A[0]);
+        const double DTKD = (newton_h(A, TKD) - h0) / den;
         if (fabs(DTKD) <= (double)0.001f) { *conv = true; break; }
         TKD = TKD - DTKD;
     }
     if (TKD > UC_TPOL2) TKD = UC_TPOL2;
     if (TKD < P.TKDMIN) TKD = P.TKDMIN;
     return TKD / P.TSTR;
+}
+
+// rho of an ideal gas at p / PSTR = pnd (main:1056-1062)
+__device__ __forceinline__ double gas_density(const DevParams &P, double tk, double pnd, const double *y, int ys)
+{
+    double r0 = 0.0, r1 = 0.0;
+#pragma unroll
+    for (int k = 0; k < LSP; k += 2) {
+        r0 = CO_FMA(__ldg(P.tbw + k), y[k * ys], r0);
+        r1 = CO_FMA(__ldg(P.tbw + k + 1), y[(k + 1) * ys], r1);
+    }
+    return pnd / (P.BETA1 * tk * (r0 + r1));
 }
 
 // Sub-step count per cell from the omega of the start state (QDSP rows):
@@ -239,25 +259,25 @@ __global__ void temperature_held_kernel(const DevParams *Pp, const double *enth,
         bool conv;
         const double t = temperature_at(P, tk[c], y + c, npad, enth[c], &conv);
         if (!conv && status) atomicCAS(status, ST_OK, ST_NEWTON_NOCONV);
-        double rbar = 0.0;
-        for (int k = 0; k < LSP; ++k) rbar = rbar + y[(size_t)k * npad + c] / P.WM[k];
         tk[c] = t;
-        rho[c] = pnd[c] / (P.BETA1 * t * rbar);
+        rho[c] = gas_density(P, t, pnd[c], y + c, npad);
     }
 }
 
 // ---- stable counting sort of positions by n_sub, largest first.
-// Chunk j of SORT_CHUNK cells is owned by CTA j; key = nsub_max - n_sub.
-constexpr int SORT_CHUNK = 4096;
+// Chunk j of `chunk` cells is owned by CTA j; key = nsub_max - n_sub. A chunk is scattered by one warp, 32 cells
+// after 32 (67 us for 4096 cells, 14 us for 512), so small fields have small chunks; up to 256 of them, which one CTA scans.
+// The order does not depend on the chunks.
+__host__ __device__ constexpr int sort_chunk(int n) { return n <= 256 * 512 ? 512 : n <= 256 * 2048 ? 2048 : 4096; }
 constexpr int SORT_MAXBIN = 1024;
 
-__global__ void sort_count_kernel(const int *nsub, int n, int nsub_max, int nchunk, int *hist)
+__global__ void sort_count_kernel(const int *nsub, int n, int nsub_max, int chunk, int nchunk, int *hist)
 {
     __shared__ int h[SORT_MAXBIN + 1];
     const int j = blockIdx.x;
     for (int b = threadIdx.x; b <= nsub_max; b += blockDim.x) h[b] = 0;
     __syncthreads();
-    const int c0 = j * SORT_CHUNK, c1 = min(n, c0 + SORT_CHUNK);
+    const int c0 = j * chunk, c1 = min(n, c0 + chunk);
     for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) atomicAdd(&h[nsub_max - nsub[c]], 1);
     __syncthreads();
     for (int b = threadIdx.x; b <= nsub_max; b += blockDim.x) hist[(size_t)b * nchunk + j] = h[b];
@@ -295,14 +315,14 @@ __global__ void sort_scan_kernel(int *hist, int total)
 }
 
 // Scatter: one warp per chunk walks its cells in index order (stable).
-__global__ void sort_scatter_kernel(const int *nsub, int n, int npad, int nsub_max, int nchunk, const int *offs,
+__global__ void sort_scatter_kernel(const int *nsub, int n, int npad, int nsub_max, int chunk, int nchunk, const int *offs,
                                     int *order)
 {
     __shared__ int off[SORT_MAXBIN + 1];
     const int j = blockIdx.x, lane = threadIdx.x;
     for (int b = lane; b <= nsub_max; b += 32) off[b] = offs[(size_t)b * nchunk + j];
     __syncwarp();
-    const int c0 = j * SORT_CHUNK, c1 = min(n, c0 + SORT_CHUNK);
+    const int c0 = j * chunk, c1 = min(n, c0 + chunk);
     for (int base = c0; base < c1; base += 32) {
         const int c = base + lane;
         const bool v = c < c1;
@@ -378,28 +398,28 @@ __global__ void round_key_kernel(const int *nsub, const int *last, const int *nl
         key[pos] = nsub[pos] > r + 1 ? 100 - min(max(last[pos], 1), 100) : ROUND_KEYS - 1;
 }
 
-// Stable counting sort of the first *nlive keys (chunks of SORT_CHUNK; hist [nbins][nchunk], scanned by
+// Stable counting sort of the first *nlive keys (chunks of sort_chunk(n); hist [nbins][nchunk], scanned by
 // sort_scan_kernel in between): perm[new position] = old position.
-__global__ void key_count_kernel(const int *key, const int *nlive, int nbins, int nchunk, int *hist)
+__global__ void key_count_kernel(const int *key, const int *nlive, int nbins, int chunk, int nchunk, int *hist)
 {
     __shared__ int h[SORT_MAXBIN];
     const int j = blockIdx.x, n = *nlive;
     for (int b = threadIdx.x; b < nbins; b += blockDim.x) h[b] = 0;
     __syncthreads();
-    const int c0 = j * SORT_CHUNK, c1 = min(n, c0 + SORT_CHUNK);
+    const int c0 = j * chunk, c1 = min(n, c0 + chunk);
     for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) atomicAdd(&h[key[c]], 1);
     __syncthreads();
     for (int b = threadIdx.x; b < nbins; b += blockDim.x) hist[(size_t)b * nchunk + j] = h[b];
 }
 
-__global__ void key_scatter_kernel(const int *key, const int *nlive, int nbins, int nchunk, const int *offs,
+__global__ void key_scatter_kernel(const int *key, const int *nlive, int nbins, int chunk, int nchunk, const int *offs,
                                    int *perm)
 {
     __shared__ int off[SORT_MAXBIN];
     const int j = blockIdx.x, lane = threadIdx.x, n = *nlive;
     for (int b = lane; b < nbins; b += 32) off[b] = offs[(size_t)b * nchunk + j];
     __syncwarp();
-    const int c0 = j * SORT_CHUNK, c1 = min(n, c0 + SORT_CHUNK);
+    const int c0 = j * chunk, c1 = min(n, c0 + chunk);
     for (int base = c0; base < c1; base += 32) {
         const int c = base + lane;
         const bool v = c < c1;
@@ -416,24 +436,28 @@ __global__ void key_scatter_kernel(const int *key, const int *nlive, int nbins, 
     }
 }
 
-// d[pos] = s[perm[pos]] for the first *nlive positions, d[pos] = s[pos] beyond
+// d[pos] = s[perm[pos]] for the first *nlive positions, d[pos] = s[pos] beyond; blockIdx.y: one of the Y rows or,
+// last, the other values
+constexpr int PERMUTE_ROWS = LSP + 1;
 __global__ void permute_state_kernel(const int *perm, const int *nlive, int npad, RoundState s, RoundState d)
 {
-    const int n = *nlive;
-    for (int pos = blockIdx.x * blockDim.x + threadIdx.x; pos < npad; pos += gridDim.x * blockDim.x) {
-        const int q = pos < n ? perm[pos] : pos;
-        for (int k = 0; k < LSP; ++k) d.y[(size_t)k * npad + pos] = s.y[(size_t)k * npad + q];
-        d.tk[pos] = s.tk[q];
-        d.rho[pos] = s.rho[q];
-        d.pnd[pos] = s.pnd[q];
-        d.soot[pos] = s.soot[q];
-        d.soot[npad + pos] = s.soot[npad + q];
-        d.enth[pos] = s.enth[q];
-        d.nsub[pos] = s.nsub[q];
-        d.passes[pos] = s.passes[q];
-        d.last[pos] = s.last[q];
-        d.ord[pos] = s.ord[q];
+    const int pos = blockIdx.x * blockDim.x + threadIdx.x;
+    if (pos >= npad) return;
+    const int q = pos < *nlive ? perm[pos] : pos;
+    if (blockIdx.y < LSP) {
+        d.y[(size_t)blockIdx.y * npad + pos] = s.y[(size_t)blockIdx.y * npad + q];
+        return;
     }
+    d.tk[pos] = s.tk[q];
+    d.rho[pos] = s.rho[q];
+    d.pnd[pos] = s.pnd[q];
+    d.soot[pos] = s.soot[q];
+    d.soot[npad + pos] = s.soot[npad + q];
+    d.enth[pos] = s.enth[q];
+    d.nsub[pos] = s.nsub[q];
+    d.passes[pos] = s.passes[q];
+    d.last[pos] = s.last[q];
+    d.ord[pos] = s.ord[q];
 }
 
 // back to cell order (the first n positions)
@@ -690,9 +714,7 @@ __global__ void __launch_bounds__(NW * 32, 1) integrate_fp64_kernel(const IntArg
                 bool conv;
                 tk = temperature_at(P, tk, sY + lane, TILE, ENTH0, &conv);
                 tconv = tconv && conv;
-                double rbar = 0.0;
-                for (int k = 0; k < LSP; ++k) rbar = rbar + sY[k * TILE + lane] / P.WM[k];
-                rho = pnd / (P.BETA1 * tk * rbar);
+                rho = gas_density(P, tk, pnd, sY + lane, TILE);
             }
             __syncthreads();
         }

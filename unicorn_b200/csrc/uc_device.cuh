@@ -81,6 +81,8 @@ struct DevParams {
     // (b, k) at b * LSP + k: 1 / WMCD, WMIK(k, b), 1 / DWMIK(k, b) (RETLJ1 is symmetric)
     double prow[2][PROP_ROWS][LSP];
     double piw[LSP * LSP], pw[LSP * LSP], pid[LSP * LSP];
+    // per temperature range and species the coefficients of A1..A6 of the T Newton: p_i / W_k / (i + 1), and p_6 / W_k
+    alignas(16) double tco[2][LSP][6];
     // third bodies as weights of Y: row 0 TBODY (1 / W_k), rows 1..10 the groups
     double tbw[11 * LSP];
     // third-body groups 1..10 (TBODY + sum sign*coef*Y/W)

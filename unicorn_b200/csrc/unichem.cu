@@ -263,6 +263,9 @@ static void build_params(const uc_inputs &in, DevParams &P, std::vector<uint8_t>
             P.ETLJ4[ij] = P.ETLJ3[ij] * P.ETLJ1[ij];
             P.RETLJ1[ij] = 1.0 / P.ETLJ1[ij];
         }
+    for (int r = 0; r < 2; ++r)
+        for (int k = 0; k < LSP; ++k)
+            for (int i = 0; i < 6; ++i) P.tco[r][k][i] = uc_poly[k * 14 + 7 * r + i] / P.WM[k] / (i < 5 ? i + 1.0 : 1.0);
     for (int r = 0; r < 2; ++r)         // the property kernel's tables
         for (int k = 0; k < LSP; ++k) {
             auto row = [&](int i) -> double & { return P.prow[r][i][k]; };
@@ -1821,7 +1824,7 @@ static int ensure_pressure(uc_ctx *ctx)
 static int integrate_buffers(uc_ctx *ctx)
 {
     const size_t np = ctx->npad;
-    const int nchunk = (ctx->n + SORT_CHUNK - 1) / SORT_CHUNK;
+    const int chunk = sort_chunk(ctx->n), nchunk = (ctx->n + chunk - 1) / chunk;
     RET_IF(ensure_pressure(ctx));
     RET_IF(dalloc(ctx, &ctx->qdsp, (size_t)LSP * np));
     int **bufs[] = {&ctx->nsub, &ctx->order, &ctx->cpasses, &ctx->hist, &ctx->next_tile};
@@ -1865,7 +1868,7 @@ extern "C" int uc_temperature_from_held(uc_ctx *ctx)
     RET_IF(ensure_pressure(ctx));
     int slot;
     prof_begin(ctx, UC_K_TEMP, slot);
-    temperature_held_kernel<<<ctx->nsm * 4, 128, 0, ctx->stream>>>(ctx->dP, ctx->enth, ctx->y, ctx->pnd, ctx->npad,
+    temperature_held_kernel<<<(ctx->npad + 63) / 64, 64, 0, ctx->stream>>>(ctx->dP, ctx->enth, ctx->y, ctx->pnd, ctx->npad,
                                                                     ctx->tk, ctx->rho, ctx->status);
     prof_end(ctx, slot);
     CK(cudaGetLastError());
@@ -1918,7 +1921,7 @@ static int *round_tile_list(uc_ctx *ctx) { return round_tiles(ctx) + SORT_MAXBIN
 static int enqueue_rounds(uc_ctx *ctx, const uc_integrate_opts &o)
 {
     const int np = ctx->npad;
-    const int nchunk = (ctx->n + SORT_CHUNK - 1) / SORT_CHUNK;
+    const int chunk = sort_chunk(ctx->n), nchunk = (ctx->n + chunk - 1) / chunk;
     int *cells = round_cells(ctx), *tiles = round_tiles(ctx), *key = round_key(ctx), *perm = round_perm(ctx);
     const int eg = std::max(1, std::min((np + 255) / 256, ctx->nsm * 8));
     round_counts_kernel<<<(o.nsub_max + 255) / 256, 256, 0, ctx->stream>>>(ctx->hist, nchunk, o.nsub_max, cells, tiles);
@@ -1949,19 +1952,19 @@ static int enqueue_rounds(uc_ctx *ctx, const uc_integrate_opts &o)
                                                                                rs.last, ctx->status, ctx->tr_map[0],
                                                                                ctx->tr_map[1]);
         CK(cudaGetLastError());
-        temperature_held_kernel<<<ctx->nsm * 4, 128, 0, ctx->stream>>>(ctx->dP, rs.enth, rs.y, rs.pnd, np, rs.tk,
+        temperature_held_kernel<<<(np + 63) / 64, 64, 0, ctx->stream>>>(ctx->dP, rs.enth, rs.y, rs.pnd, np, rs.tk,
                                                                         rs.rho, ctx->status, cells + r);
         CK(cudaGetLastError());
         if (r + 1 == o.nsub_max) break;
         round_key_kernel<<<eg, 256, 0, ctx->stream>>>(rs.nsub, rs.last, cells + r, r, key);
         CK(cudaGetLastError());
-        key_count_kernel<<<nchunk, 256, 0, ctx->stream>>>(key, cells + r, ROUND_KEYS, nchunk, ctx->hist);
+        key_count_kernel<<<nchunk, 256, 0, ctx->stream>>>(key, cells + r, ROUND_KEYS, chunk, nchunk, ctx->hist);
         CK(cudaGetLastError());
         sort_scan_kernel<<<1, 1024, 0, ctx->stream>>>(ctx->hist, ROUND_KEYS * nchunk);
         CK(cudaGetLastError());
-        key_scatter_kernel<<<nchunk, 32, 0, ctx->stream>>>(key, cells + r, ROUND_KEYS, nchunk, ctx->hist, perm);
+        key_scatter_kernel<<<nchunk, 32, 0, ctx->stream>>>(key, cells + r, ROUND_KEYS, chunk, nchunk, ctx->hist, perm);
         CK(cudaGetLastError());
-        permute_state_kernel<<<eg, 256, 0, ctx->stream>>>(perm, cells + r, np, rs, other);
+        permute_state_kernel<<<dim3((np + 255) / 256, PERMUTE_ROWS), 256, 0, ctx->stream>>>(perm, cells + r, np, rs, other);
         CK(cudaGetLastError());
         std::swap(rs, other);
     }
@@ -2002,12 +2005,12 @@ static int enqueue_integrate(uc_ctx *ctx, int precision, const uc_integrate_opts
         ctx->dP, ctx->rho, ctx->y, ctx->qdsp, ctx->n, np, o.dt, o.c_tau, o.y_tau, o.nsub_max, ctx->nsub);
     CK(cudaGetLastError());
     if (sorted) {
-        const int nchunk = (ctx->n + SORT_CHUNK - 1) / SORT_CHUNK;
-        sort_count_kernel<<<nchunk, 256, 0, ctx->stream>>>(ctx->nsub, ctx->n, o.nsub_max, nchunk, ctx->hist);
+        const int chunk = sort_chunk(ctx->n), nchunk = (ctx->n + chunk - 1) / chunk;
+        sort_count_kernel<<<nchunk, 256, 0, ctx->stream>>>(ctx->nsub, ctx->n, o.nsub_max, chunk, nchunk, ctx->hist);
         CK(cudaGetLastError());
         sort_scan_kernel<<<1, 1024, 0, ctx->stream>>>(ctx->hist, (o.nsub_max + 1) * nchunk);
         CK(cudaGetLastError());
-        sort_scatter_kernel<<<nchunk, 32, 0, ctx->stream>>>(ctx->nsub, ctx->n, np, o.nsub_max, nchunk, ctx->hist,
+        sort_scatter_kernel<<<nchunk, 32, 0, ctx->stream>>>(ctx->nsub, ctx->n, np, o.nsub_max, chunk, nchunk, ctx->hist,
                                                            ctx->order);
         CK(cudaGetLastError());
     }
