@@ -302,6 +302,7 @@ __global__ void splitk_reduce_kernel(const float *part, int splits, int M, int N
     const size_t mn = (size_t)M * N;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < mn; i += (size_t)gridDim.x * blockDim.x) {
         float acc = 0.0f;
+#pragma unroll 16
         for (int z = 0; z < splits; ++z) acc += part[(size_t)z * mn + i];
         out[(i / N) * ldo + i % N] = acc;
     }

@@ -2354,6 +2354,10 @@ constexpr size_t MLP_WS_FLOATS = (size_t)32 * MLP_H * MLP_H;
 struct uc_mlp {
     int device = 0;
     cudaStream_t stream = nullptr;
+    // the weight gradients beside the gradient's way down the layers: their own stream, forked from and joined to
+    // `stream` by events (in the captured step: a parallel branch of the graph)
+    cudaStream_t side = nullptr;
+    cudaEvent_t ready[MLP_LAYERS] = {}, joined = nullptr;
     MlpNorm hnorm{};
     MlpNorm *dnorm = nullptr;
     bool have_norm = false;
@@ -2430,8 +2434,13 @@ extern "C" int uc_mlp_create(int device, unsigned long long seed, long capacity,
     uc_mlp *mlp = new (std::nothrow) uc_mlp();
     if (!mlp) return UC_E_NOMEM;
     mlp->device = device;
-    if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&mlp->stream, cudaStreamNonBlocking) != cudaSuccess) {
-        delete mlp;
+    bool made = cudaSetDevice(device) == cudaSuccess &&
+                cudaStreamCreateWithFlags(&mlp->stream, cudaStreamNonBlocking) == cudaSuccess &&
+                cudaStreamCreateWithFlags(&mlp->side, cudaStreamNonBlocking) == cudaSuccess &&
+                cudaEventCreateWithFlags(&mlp->joined, cudaEventDisableTiming) == cudaSuccess;
+    for (auto &e : mlp->ready) made = made && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+    if (!made) {
+        uc_mlp_destroy(mlp);
         return UC_E_CUDA;
     }
     int off = 0, bo = 0;
@@ -2640,25 +2649,29 @@ static int mlp_enqueue_fwd_bwd(uc_mlp *mlp, int B, float *loss_hist)
     const int lblk = 256;
     mlp_loss_grad_kernel<<<lblk, 256, 0, st>>>(mlp->Out, mlp->T, B, mlp->G[MLP_LAYERS - 1], mlp->partial);
     MCK(cudaGetLastError());
-    if (loss_hist) {
-        mlp_loss_final_kernel<<<1, 32, 0, st>>>(mlp->partial, lblk, B, mlp->d_iter, loss_hist);
-        MCK(cudaGetLastError());
-    }
     for (int l = MLP_LAYERS - 1; l >= 0; --l) {
         const int in = mlp->in[l], out = mlp->out[l];
-        dim3 tb(32, 8);
-        transpose_bf16_kernel<<<dim3((out + 31) / 32, (B + 31) / 32), tb, 0, st>>>(mlp->G[l], B, out, mlp->Gt);
-        transpose_bf16_kernel<<<dim3((in + 31) / 32, (B + 31) / 32), tb, 0, st>>>(mlp->H[l], B, in, mlp->Ht);
+        // G[l] is ready: its weight gradient on the side stream (Gt, Ht and ws are that stream's alone)
+        MCK(cudaEventRecord(mlp->ready[l], st));
+        MCK(cudaStreamWaitEvent(mlp->side, mlp->ready[l], 0));
+        if (l == MLP_LAYERS - 1 && loss_hist) {
+            mlp_loss_final_kernel<<<1, 32, 0, mlp->side>>>(mlp->partial, lblk, B, mlp->d_iter, loss_hist);
+            MCK(cudaGetLastError());
+        }
+        transpose_bf16_kernel<<<dim3((std::max(in, out) + 63) / 64, (B + 63) / 64, 2), dim3(32, 8), 0, mlp->side>>>(
+            mlp->G[l], out, mlp->Gt, mlp->H[l], in, mlp->Ht, B);
         MCK(cudaGetLastError());
         // dW[out][in] = G^T H over the batch
-        RET_IF(mlp_gemm(mlp, st, mlp->Gt, B, mlp->Ht, B, out, in, B, EPI_F32, nullptr, nullptr, nullptr, 0,
+        RET_IF(mlp_gemm(mlp, mlp->side, mlp->Gt, B, mlp->Ht, B, out, in, B, EPI_F32, nullptr, nullptr, nullptr, 0,
                         mlp->g + mlp->woff[l], nullptr, in));
-        bias_grad_kernel<<<(out + 7) / 8, 256, 0, st>>>(mlp->Gt, B, out, mlp->g + mlp->boff[l]);
+        bias_grad_kernel<<<(out + 1) / 2, 64, 0, mlp->side>>>(mlp->Gt, B, out, mlp->g + mlp->boff[l]);
         MCK(cudaGetLastError());
         if (l > 0)   // gradient w.r.t. the previous pre-activation: (G W) * gelu'(z)
             RET_IF(mlp_gemm(mlp, st, mlp->G[l], out, mlp->wbt + mlp->bfoff[l], out, B, in, out, EPI_DGELU, nullptr,
                             mlp->Z[l - 1], nullptr, MLP_H, nullptr, mlp->G[l - 1], in));
     }
+    MCK(cudaEventRecord(mlp->joined, mlp->side));
+    MCK(cudaStreamWaitEvent(st, mlp->joined, 0));
     return UC_OK;
 }
 
@@ -2925,6 +2938,7 @@ extern "C" void uc_mlp_destroy(uc_mlp *mlp)
     if (!mlp) return;
     cudaSetDevice(mlp->device);
     if (mlp->stream) cudaStreamSynchronize(mlp->stream);
+    if (mlp->side) cudaStreamSynchronize(mlp->side);
     if (mlp->train_exec) cudaGraphExecDestroy(mlp->train_exec);
     if (mlp->train_graph) cudaGraphDestroy(mlp->train_graph);
     void *bufs[] = {mlp->dnorm, mlp->w, mlp->g, mlp->m, mlp->v, mlp->wb, mlp->wbt, mlp->Xall, mlp->Tall,
@@ -2935,6 +2949,10 @@ extern "C" void uc_mlp_destroy(uc_mlp *mlp)
         if (b) cudaFree(b);
     mlp_free_batch(mlp);
     if (mlp->sample) uc_destroy(mlp->sample);
+    for (auto e : mlp->ready)
+        if (e) cudaEventDestroy(e);
+    if (mlp->joined) cudaEventDestroy(mlp->joined);
+    if (mlp->side) cudaStreamDestroy(mlp->side);
     if (mlp->stream) cudaStreamDestroy(mlp->stream);
     delete mlp;
 }
