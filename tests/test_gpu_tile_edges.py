@@ -73,3 +73,32 @@ def test_props_and_cp_h_at_tile_edges(cuda, oracle, n):
     assert_rel(cp, oracle.cp(tk, yo), 1e-11, 0, "cp")
     hm = oracle.enthalpy(tk, yo)[1]
     assert_rel(h, hm, 1e-10, 1e-12 * np.abs(hm).max(), "h")
+
+
+@pytest.mark.parametrize("n", [1, 31, 512, 513])
+def test_host_copies_on_both_sides_of_the_staged_size(cuda, oracle, n):
+    """Fields of up to 512 cells pass through pinned staging rows. The caller's arrays may be overwritten as soon
+    as upload returns, uploads may follow one another, and what comes back is what went in."""
+    rng = np.random.default_rng(n)
+    states = [(rng.uniform(1, 8, n), rng.uniform(0.1, 1, n), rng.uniform(0, 1, (52, n)), rng.uniform(0, 1e-3, n),
+               rng.uniform(0, 1e12, n)) for _ in range(3)]
+    with cuda.UniChem(n) as u:
+        for st in states:
+            work = [a.copy() for a in st]
+            u.upload(*work)
+            for a in work:
+                a[...] = -1.0
+        for a, b in zip(u.download(), states[-1]):
+            assert np.array_equal(a, b)
+        u.upload(*states[0][:3])                      # without soot: zeros
+        got = u.download()
+        assert np.array_equal(got[2], states[0][2]) and not got[3].any() and not got[4].any()
+        with pytest.raises(cuda.UniChemError):
+            u.download_outputs()                      # nothing computed yet
+        tk, rho, y = random_state(oracle, n, 5)
+        u.upload(tk, rho, y)
+        om, (mu, lam, d) = u.omega(), u.props()
+        cp, h = u.cp_h()
+        o = u.download_outputs()
+    for k, v in dict(qdsp=om.qdsp, qdot=om.qdot, domega_dy=om.domega_dy, vmu=mu, vtc=lam, vdf=d, cp=cp, h=h).items():
+        assert np.array_equal(o[k], v), k

@@ -49,6 +49,10 @@ struct uc_ctx {
     cudaStream_t stream = nullptr;
     cudaStream_t io_stream = nullptr;  // uc_sweep_host: copies of the outputs while the update runs
     cudaEvent_t io_event = nullptr;
+    // fields of up to STAGE_CELLS cells: pinned staging of the host copies (upload rows, then download rows and
+    // the status word), read and written by one kernel each; null for larger fields
+    double *stage = nullptr;
+    cudaEvent_t stage_read = nullptr;  // the last upload kernel has read its rows
     uc_scales sc{};
     uc_inputs inputs{};               // the input-card values of uc_init
     DevParams *hP = nullptr;          // host copy
@@ -154,6 +158,12 @@ static int set_err(uc_ctx *c, int code, const char *fmt, ...)
         if (e_ != cudaSuccess)                                                                   \
             return set_err(ctx, UC_E_CUDA, "%s failed: %s (%s:%d)", #call, cudaGetErrorString(e_), \
                            __FILE__, __LINE__);                                                  \
+    } while (0)
+
+#define RET_IF(x)                 \
+    do {                          \
+        int r_ = (x);             \
+        if (r_ != UC_OK) return r_; \
     } while (0)
 
 // ------------------------------------------------------------------ set-up
@@ -475,6 +485,8 @@ static void free_ctx(uc_ctx *c)
     }
     for (auto e : c->ev_pool) cudaEventDestroy(e);
     c->ev_pool.clear();
+    if (c->stage) cudaFreeHost(c->stage);
+    if (c->stage_read) cudaEventDestroy(c->stage_read);
     if (c->stream) cudaStreamDestroy(c->stream);
     if (c->io_stream) cudaStreamDestroy(c->io_stream);
     if (c->io_event) cudaEventDestroy(c->io_event);
@@ -545,6 +557,78 @@ static int check_status(uc_ctx *ctx)
     return UC_OK;
 }
 
+// Host copies of a small field. A pageable copy costs 8-10 us whatever its size, and an upload has eleven copies,
+// fills and pad launches, a download up to four copies and a wait: for a few hundred cells those calls were
+// most of the time (one cell, upload and omega: 131 us, of which 28 the rate kernel; 62 us this way). Up to STAGE_CELLS cells the host rows
+// go through pinned memory that one kernel reads or writes in place; beyond, the copies' bandwidth decides and
+// they stay.
+constexpr int STAGE_CELLS = 512;
+constexpr int STAGE_UP = LSP + 4, STAGE_DOWN = 3 * LSP + 5;       // rows: tk, rho, Y, soot; the most a call returns
+
+__global__ void stage_upload_kernel(const double *stage, int n, int npad, double *tk, double *rho, double *y, double *y0,
+                                    double *soot, double *soot0)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < STAGE_UP * npad; i += gridDim.x * blockDim.x) {
+        const int r = i / npad, c = i % npad;
+        const double v = stage[(size_t)r * n + min(c, n - 1)];    // the padding cells copy the last cell
+        if (r == 0) tk[c] = v;
+        else if (r == 1) rho[c] = v;
+        else if (r < LSP + 2) y[(size_t)(r - 2) * npad + c] = y0[(size_t)(r - 2) * npad + c] = v;
+        else soot[(size_t)(r - LSP - 2) * npad + c] = soot0[(size_t)(r - LSP - 2) * npad + c] = v;
+    }
+}
+
+struct StageRows {
+    const double *src[8];
+    int rows[8], parts;
+};
+__global__ void stage_download_kernel(const StageRows s, int n, int npad, const int *status, double *stage)
+{
+    size_t base = 0;
+    for (int p = 0; p < s.parts; ++p) {
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < s.rows[p] * n; i += gridDim.x * blockDim.x)
+            stage[base + i] = s.src[p][(size_t)(i / n) * npad + i % n];
+        base += (size_t)s.rows[p] * n;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<int *>(stage + base) = *status;
+}
+
+// Rows of device arrays to host arrays (null destinations are left out), and the wait for them; with_status: and
+// the status the kernels left (check_status).
+struct DownRows { double *dst; const double *src; int rows; };
+static int download_parts(uc_ctx *ctx, const DownRows *d, int nd, bool with_status)
+{
+    StageRows s{};
+    int rows = 0;
+    for (int i = 0; i < nd; ++i)
+        if (d[i].dst) {
+            if (s.parts < 8) {
+                s.src[s.parts] = d[i].src;
+                s.rows[s.parts] = d[i].rows;
+            }
+            ++s.parts;
+            rows += d[i].rows;
+        }
+    if (!ctx->stage || s.parts > 8 || rows > STAGE_DOWN) {
+        for (int i = 0; i < nd; ++i) RET_IF(download_rows(ctx, d[i].dst, d[i].src, d[i].rows));
+        if (with_status) return check_status(ctx);
+        CK(cudaStreamSynchronize(ctx->stream));
+        return UC_OK;
+    }
+    double *down = ctx->stage + (size_t)STAGE_UP * ctx->n;
+    stage_download_kernel<<<std::max(1, std::min((rows * ctx->n + 255) / 256, 2 * ctx->nsm)), 256, 0, ctx->stream>>>(
+        s, ctx->n, ctx->npad, ctx->status, down);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(ctx->stream));
+    for (int i = 0; i < nd; ++i)
+        if (d[i].dst) {
+            memcpy(d[i].dst, down, (size_t)d[i].rows * ctx->n * sizeof(double));
+            down += (size_t)d[i].rows * ctx->n;
+        }
+    if (with_status && *reinterpret_cast<const int *>(down) != ST_OK) return check_status(ctx);
+    return UC_OK;
+}
+
 // Species update with Y in place: 14 warps per CTA (one CTA per SM). Measured on
 // the C2 sweep against the two-Y-set kernel at 8 warps: 0.56 against 0.65 ms
 // per pass; 12, 16 and 17 warps gave 0.62, 0.57 and 0.66 (fewer registers per
@@ -607,12 +691,6 @@ static const void *tr_kernel(bool faces)
     return faces ? (const void *)update_tr_kernel<true> : (const void *)update_tr_kernel<false>;
 }
 
-#define RET_IF(x)                 \
-    do {                          \
-        int r_ = (x);             \
-        if (r_ != UC_OK) return r_; \
-    } while (0)
-
 // ------------------------------------------------------------------ C ABI
 
 extern "C" int uc_init(const uc_inputs *in, int ncell, int device, uc_ctx **out)
@@ -630,9 +708,8 @@ extern "C" int uc_init(const uc_inputs *in, int ncell, int device, uc_ctx **out)
         cudaError_t e = cudaSetDevice(device);
         if (e != cudaSuccess) { rc = set_err(ctx, UC_E_CUDA, "cudaSetDevice(%d): %s", device, cudaGetErrorString(e)); break; }
         ctx->device = device;
-        cudaDeviceProp prop;
-        cudaGetDeviceProperties(&prop, device);
-        ctx->nsm = prop.multiProcessorCount;
+        e = cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, device);
+        if (e != cudaSuccess) { rc = set_err(ctx, UC_E_CUDA, "device attribute: %s", cudaGetErrorString(e)); break; }
         e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
         if (e != cudaSuccess) { rc = set_err(ctx, UC_E_CUDA, "stream: %s", cudaGetErrorString(e)); break; }
         ctx->n = ncell;
@@ -664,6 +741,13 @@ extern "C" int uc_init(const uc_inputs *in, int ncell, int device, uc_ctx **out)
             (rc = dalloc(ctx, &ctx->sour, 6 * np)))
             break;
         cudaMemset(ctx->sour, 0, 6 * np * sizeof(double));
+        if (ncell <= STAGE_CELLS &&
+            (cudaEventCreateWithFlags(&ctx->stage_read, cudaEventDisableTiming) != cudaSuccess ||
+             cudaHostAlloc((void **)&ctx->stage, ((size_t)(STAGE_UP + STAGE_DOWN) * ncell + 1) * sizeof(double),
+                           cudaHostAllocDefault) != cudaSuccess)) {
+            ctx->stage = nullptr;             // without it the copies of larger fields serve
+            cudaGetLastError();
+        }
         e = cudaFuncSetAttribute(chem_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CHEM_SMEM);
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(chem_mixed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CHEMM_SMEM);
@@ -749,6 +833,28 @@ extern "C" int uc_upload_fields(uc_ctx *ctx, const double *tk, const double *rho
 {
     if (!ctx || !tk || !rho || !fsp) return set_err(ctx, UC_E_ARG, "uc_upload_fields: tk, rho and fsp are required");
     CK(cudaSetDevice(ctx->device));
+    if (ctx->stage) {
+        CK(cudaEventSynchronize(ctx->stage_read));      // the last upload has left the staging rows
+        const size_t row = (size_t)ctx->n * sizeof(double);
+        double *s = ctx->stage;
+        memcpy(s, tk, row);
+        memcpy(s + ctx->n, rho, row);
+        memcpy(s + 2 * (size_t)ctx->n, fsp, LSP * row);
+        s += (size_t)(LSP + 2) * ctx->n;
+        const double *soot[2] = {stmf, stnd};
+        for (int i = 0; i < 2; ++i, s += ctx->n) {
+            if (soot[i]) memcpy(s, soot[i], row);
+            else memset(s, 0, row);
+        }
+        stage_upload_kernel<<<std::min((STAGE_UP * ctx->npad + 255) / 256, 2 * ctx->nsm), 256, 0, ctx->stream>>>(
+            ctx->stage, ctx->n, ctx->npad, ctx->tk, ctx->rho, ctx->y, ctx->y0, ctx->soot, ctx->soot0);
+        CK(cudaGetLastError());
+        CK(cudaEventRecord(ctx->stage_read, ctx->stream));
+        ctx->have_fields = true;
+        ctx->have_rc = false;
+        ctx->rc_start = false;
+        return UC_OK;
+    }
     RET_IF(upload_rows(ctx, ctx->tk, tk, 1));
     RET_IF(upload_rows(ctx, ctx->rho, rho, 1));
     RET_IF(upload_rows(ctx, ctx->y, fsp, LSP));
@@ -859,13 +965,9 @@ extern "C" int uc_download_fields(uc_ctx *ctx, double *tk, double *rho, double *
     if (!ctx) return UC_E_ARG;
     if (!ctx->have_fields) return set_err(ctx, UC_E_STATE, "no fields uploaded");
     CK(cudaSetDevice(ctx->device));
-    RET_IF(download_rows(ctx, tk, ctx->tk, 1));
-    RET_IF(download_rows(ctx, rho, ctx->rho, 1));
-    RET_IF(download_rows(ctx, fsp, ctx->y, LSP));
-    RET_IF(download_rows(ctx, stmf, ctx->soot, 1));
-    RET_IF(download_rows(ctx, stnd, ctx->soot + ctx->npad, 1));
-    CK(cudaStreamSynchronize(ctx->stream));
-    return UC_OK;
+    const DownRows d[] = {{tk, ctx->tk, 1}, {rho, ctx->rho, 1}, {fsp, ctx->y, LSP}, {stmf, ctx->soot, 1},
+                          {stnd, ctx->soot + ctx->npad, 1}};
+    return download_parts(ctx, d, 5, false);
 }
 
 static int launch_chem(uc_ctx *ctx, int precision, bool want_rc, bool want_omega)
@@ -996,10 +1098,8 @@ extern "C" int uc_omega(uc_ctx *ctx, int precision, double *qdsp, double *qdot, 
     CK(cudaSetDevice(ctx->device));
     RET_IF(launch_chem(ctx, precision, false, true));
     if (qdsp || qdot || domega_dy) {
-        RET_IF(download_rows(ctx, qdsp, ctx->qdsp, LSP));
-        RET_IF(download_rows(ctx, qdot, ctx->qdot, 1));
-        RET_IF(download_rows(ctx, domega_dy, ctx->dwdy, LSP));
-        RET_IF(check_status(ctx));
+        const DownRows d[] = {{qdsp, ctx->qdsp, LSP}, {qdot, ctx->qdot, 1}, {domega_dy, ctx->dwdy, LSP}};
+        RET_IF(download_parts(ctx, d, 3, true));
     }
     return UC_OK;
 }
@@ -1024,10 +1124,8 @@ static int props_impl(uc_ctx *ctx, int precision, double *vmu, double *vtc, doub
     prof_end(ctx, slot);
     CK(cudaGetLastError());
     if (vmu || vtc || vdf) {
-        RET_IF(download_rows(ctx, vmu, ctx->vmu, 1));
-        RET_IF(download_rows(ctx, vtc, ctx->vtc, 1));
-        RET_IF(download_rows(ctx, vdf, ctx->vdf, LSP));
-        CK(cudaStreamSynchronize(ctx->stream));
+        const DownRows d[] = {{vmu, ctx->vmu, 1}, {vtc, ctx->vtc, 1}, {vdf, ctx->vdf, LSP}};
+        RET_IF(download_parts(ctx, d, 3, false));
     }
     return UC_OK;
 }
@@ -1057,9 +1155,8 @@ static int cp_h_impl(uc_ctx *ctx, int precision, double *cp, double *h)
     prof_end(ctx, slot);
     CK(cudaGetLastError());
     if (cp || h) {
-        RET_IF(download_rows(ctx, cp, ctx->cp, 1));
-        RET_IF(download_rows(ctx, h, ctx->h, 1));
-        CK(cudaStreamSynchronize(ctx->stream));
+        const DownRows d[] = {{cp, ctx->cp, 1}, {h, ctx->h, 1}};
+        RET_IF(download_parts(ctx, d, 2, false));
     }
     return UC_OK;
 }
@@ -1286,17 +1383,16 @@ extern "C" int uc_download_outputs(uc_ctx *ctx, double *qdsp, double *qdot, doub
 {
     if (!ctx) return UC_E_ARG;
     CK(cudaSetDevice(ctx->device));
-    struct { double *dst; double *src; int rows; const char *name; } o[] = {
-        {qdsp, ctx->qdsp, LSP, "qdsp"}, {qdot, ctx->qdot, 1, "qdot"}, {domega_dy, ctx->dwdy, LSP, "domega_dy"},
-        {vmu, ctx->vmu, 1, "vmu"}, {vtc, ctx->vtc, 1, "vtc"}, {vdf, ctx->vdf, LSP, "vdf"},
-        {cp, ctx->cp, 1, "cp"}, {h, ctx->h, 1, "h"}};
-    for (auto &x : o) {
-        if (!x.dst) continue;
-        if (!x.src) return set_err(ctx, UC_E_STATE, "%s has not been computed yet", x.name);
-        RET_IF(download_rows(ctx, x.dst, x.src, x.rows));
+    const struct { DownRows d; const char *name; } o[] = {
+        {{qdsp, ctx->qdsp, LSP}, "qdsp"}, {{qdot, ctx->qdot, 1}, "qdot"}, {{domega_dy, ctx->dwdy, LSP}, "domega_dy"},
+        {{vmu, ctx->vmu, 1}, "vmu"}, {{vtc, ctx->vtc, 1}, "vtc"}, {{vdf, ctx->vdf, LSP}, "vdf"},
+        {{cp, ctx->cp, 1}, "cp"}, {{h, ctx->h, 1}, "h"}};
+    DownRows d[8];
+    for (int i = 0; i < 8; ++i) {
+        d[i] = o[i].d;
+        if (d[i].dst && !d[i].src) return set_err(ctx, UC_E_STATE, "%s has not been computed yet", o[i].name);
     }
-    CK(cudaStreamSynchronize(ctx->stream));
-    return check_status(ctx);
+    return download_parts(ctx, d, 8, true);
 }
 
 extern "C" int uc_profile(uc_ctx *ctx, int on)
