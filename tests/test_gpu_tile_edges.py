@@ -5,6 +5,9 @@ loads ahead) and one more than three per SM, against the oracle.
 The properties at the edges of theirs (8 or 16 cells a block, by the field's size) and of the sub-mixture: more
 than 32 species in it, one species alone, N2 alone.
 
+The enthalpy relaxation at the edges of its blocks of steps (8, 4, 2 or 1 by the number of rows; a number of steps
+that is or is not a multiple), bit for bit.
+
 Tolerances as in test_gpu_parity.py: mu, lambda, D_k, cp 1e-11 relative, h 1e-10; RC and d(omega)/dY 1e-11 relative; QDSP 1e-11 of the gross rate; QDOT, a
 sum of 52 products QDSP_k h_k, 1e-11 of the sum of the gross rates times |h_k|; Y after the update 1e-9."""
 import numpy as np
@@ -102,3 +105,14 @@ def test_host_copies_on_both_sides_of_the_staged_size(cuda, oracle, n):
         o = u.download_outputs()
     for k, v in dict(qdsp=om.qdsp, qdot=om.qdot, domega_dy=om.domega_dy, vmu=mu, vtc=lam, vdf=d, cp=cp, h=h).items():
         assert np.array_equal(o[k], v), k
+
+
+# interior rows for blocks of 8 (229 at most), 4 (458), 2 (916) and 1 step
+@pytest.mark.parametrize("lj,li", [(3, 10), (3, 11), (10, 3), (231, 5), (232, 6), (460, 4), (461, 4), (918, 4), (919, 3)])
+def test_relaxation_at_block_edges(cuda, oracle, lj, li):
+    from test_gpu_enthalpy import oracle_coefficients
+    g, o = oracle_coefficients(oracle, lj, li, 14)
+    fo, po = oracle.enthalpy_relax(lj, li, g["rho"], o["rhsz"], o["z"], g["ht"], isor=5, tol=-1.0)
+    fg, pg = cuda.enthalpy_relax(lj, li, g["rho"], o["rhsz"], o["z"], g["ht"], isor=5, tol=-1.0)
+    assert pg == po
+    assert np.array_equal(fg, fo)

@@ -25,8 +25,8 @@
 // ii = s - jj (a wavefront over the anti-diagonals), its west value in a
 // register and its south value from the row below through shared memory.
 // Pass p at step s reads what pass p-1 wrote at steps s and s+1, so the passes
-// run as a pipeline, two steps apart: CTA p waits for the published step count
-// of pass p-1. Pass values are stored skewed, index s*nj + jj, so the loads of
+// run as a pipeline, a block of steps and a step apart: CTA p waits for the
+// published step count of pass p-1. Pass values are stored skewed, index s*nj + jj, so the loads of
 // a step are contiguous across the rows; a ring of R pass buffers holds them.
 // A pass starts only when pass p-R+1 (the last reader of the slot it
 // overwrites) has finished. Each pass sums |dFPZ| per row in I order and then
@@ -327,18 +327,54 @@ __device__ __noinline__ int relax_wait(const int *flag, int need, int p, int *st
     }
 }
 
+// steps of a block (below), at most; and the block's length for nj rows, by shared memory: two sets of six coefficient
+// planes of that many steps
+constexpr int RELAX_BLOCK = 8;
+__host__ __device__ constexpr int relax_block(int nj)
+{
+    int b = RELAX_BLOCK;
+    while (b > 1 && 12 * b * nj > 22000) b /= 2;
+    return b;
+}
+__host__ __device__ constexpr size_t relax_smem(int nj)
+{
+    return sizeof(double) * (3 * (size_t)nj + 2 * (size_t)relax_block(nj) * (6 * (size_t)nj + 2));
+}
+
+__device__ __forceinline__ void cp_async8(double *dst, const double *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+
+// The steps run in blocks of B. What a block needs apart from the row below's new values is fetched before
+// its first step: the coefficients and the boundary values one block ahead into shared memory (cp.async), pass
+// p - 1's values into registers once that pass has published them all (one wait and one publication a block
+// instead of one a step; the passes then run up to 2 B steps apart). A step is left with the arithmetic, whose
+// chain the reference's operation order fixes, and one barrier. With the loads, the wait and the
+// publication in every step, a step took 2.9 us on a 131 x 711 grid, now 1.35 us (seven passes, 2.5 and 1.15 ms).
 __global__ void __launch_bounds__(RELAX_MAX_ROWS) enth_relax_kernel(const RelaxArgs a)
 {
     extern __shared__ __align__(16) double rsm[];
+    const int jj = threadIdx.x, nj = a.nj, ni = a.ni, B = relax_block(nj);
     double *sF = rsm;                  // [2][nj] value of the previous step, by step parity
-    double *sRow = rsm + 2 * a.nj;     // [nj] row residuals
+    double *sRow = rsm + 2 * nj;       // [nj] row residuals
+    double *sCf = sRow + nj;           // [2][6][B][nj] coefficients
+    double *sB = sCf + 2 * 6 * (size_t)B * nj;   // [2][2][B] south and north boundary values
     __shared__ int s_drop[2];
-    const int jj = threadIdx.x, nj = a.nj, ni = a.ni;
-    const bool rowthr = jj < nj;
+    const bool rowthr = jj < nj, helper = threadIdx.x == blockDim.x - 1;
     const size_t plane = (size_t)a.nstep * nj;
-    const double *cRH = a.cf + CF_RHSZ * plane, *cPP = a.cf + CF_PPP * plane, *cZN = a.cf + CF_ZN * plane;
-    const double *cZS = a.cf + CF_ZS * plane, *cZE = a.cf + CF_ZE * plane, *cZW = a.cf + CF_ZW * plane;
     const double sor1 = a.sor1, sor2 = a.sor2;
+    auto fetch = [&](int set, int s0) {
+        const int cnt = min(B, a.nstep - s0) * nj;
+        double *d = sCf + (size_t)set * 6 * B * nj;
+        for (int c = 0; c < 6; ++c)
+            for (int i = jj; i < cnt; i += blockDim.x) cp_async8(d + (size_t)c * B * nj + i, a.cf + c * plane + (size_t)s0 * nj + i);
+        if (jj < 2 * B) {              // row 0 at step s: I = s + 1; row nj - 1: I = s - nj + 2
+            const int u = jj % B, north = jj / B, ii = s0 + u - (north ? nj - 1 : 0);
+            if (ii >= 0 && ii < ni) cp_async8(sB + (set * 2 + north) * B + u, a.f0 + (size_t)(ii + 1) * a.lj + (north ? a.lj - 1 : 0));
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
     for (int p = blockIdx.x; p < a.isor; p += gridDim.x) {
         // ---- slot of this pass free (pass p-R+1 read it last) and no earlier stop
         if (threadIdx.x == 0) {
@@ -353,47 +389,70 @@ __global__ void __launch_bounds__(RELAX_MAX_ROWS) enth_relax_kernel(const RelaxA
         if (dropped_early) return;
         const double *prev = p == 0 ? a.f0s : a.ring + (size_t)((p - 1) % a.R) * plane;
         double *cur = a.ring + (size_t)(p % a.R) * plane;
-        double fw = 0.0, res = 0.0;
-        int seen = 0;                  // thread 0: steps of pass p-1 known to be published
+        fetch(0, 0);
+        // west boundary: the value left of the row's first cell; east boundary, right of its last
+        double fw = rowthr ? a.f0[jj + 1] : 0.0, res = 0.0, fold = 0.0;
+        const double feast = rowthr ? a.f0[(size_t)(a.li - 1) * a.lj + jj + 1] : 0.0;
+        int seen = 0;                  // helper: steps of pass p-1 known to be published
         bool dropped = false;
-        for (int s = 0; s < a.nstep; ++s) {
-            if (threadIdx.x == 0) {
+        for (int s0 = 0, set = 0; s0 < a.nstep; s0 += B, set ^= 1) {
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+            // steps < s0 of this pass are complete in every thread, the block's coefficients have landed
+            if (helper && s0 > 0) {
+                __threadfence();
+                st_release(a.progress + p, s0);
+            }
+            if (s0 + B < a.nstep) fetch(set ^ 1, s0 + B);
+            if (helper) {
                 int drop = 0;
-                const int need = min(s + 2, a.nstep);
+                const int need = min(s0 + B + 1, a.nstep);
                 if (p > 0 && seen < need) {
                     seen = relax_wait(a.progress + (p - 1), need, p, a.status, a.stop_at, a.timeout_ns);
                     if (seen < 0) drop = 1;
                 }
-                s_drop[s & 1] = drop;
+                s_drop[set] = drop;
             }
             __syncthreads();
-            // steps < s of this pass are complete in every thread
-            if (threadIdx.x == 0 && s > 0) {
-                __threadfence();
-                st_release(a.progress + p, s);
+            if (s_drop[set]) { dropped = true; break; }
+            // pass p - 1 east and north of the row's cells (its own value is the east one of the step before)
+            double fev[RELAX_BLOCK], fnv[RELAX_BLOCK];
+            if (s0 == 0 && rowthr) fold = __ldcg(prev + jj);
+#pragma unroll
+            for (int u = 0; u < RELAX_BLOCK; ++u) {
+                const size_t k = (size_t)(s0 + u + 1) * nj + jj;
+                const bool in = u < B && rowthr && s0 + u + 1 < a.nstep;
+                fev[u] = in ? __ldcg(prev + k) : 0.0;
+                fnv[u] = in && jj < nj - 1 ? __ldcg(prev + k + 1) : 0.0;
             }
-            if (s_drop[s & 1]) { dropped = true; break; }
-            const int ii = s - jj;
-            if (rowthr && ii >= 0 && ii < ni) {
-                const int j = jj + 1, i = ii + 1;
-                const size_t k = (size_t)s * nj + jj;
-                const double fold = __ldcg(prev + k);
-                const double fn = jj == nj - 1 ? a.f0[(size_t)i * a.lj + (a.lj - 1)] : __ldcg(prev + k + nj + 1);
-                const double fe = ii == ni - 1 ? a.f0[(size_t)(a.li - 1) * a.lj + j] : __ldcg(prev + k + nj);
-                const double fs = jj == 0 ? a.f0[(size_t)i * a.lj] : sF[((s - 1) & 1) * nj + jj - 1];
-                const double fwv = ii == 0 ? a.f0[j] : fw;
-                // FNEW = SOR2 FPZ + (RHSZ - ZN FN - ZS FS - ZE FE - ZW FW) SOR1 / PPP, rounded as written
-                double t = __dsub_rn(cRH[k], __dmul_rn(cZN[k], fn));
-                t = __dsub_rn(t, __dmul_rn(cZS[k], fs));
-                t = __dsub_rn(t, __dmul_rn(cZE[k], fe));
-                t = __dsub_rn(t, __dmul_rn(cZW[k], fwv));
-                const double fnew = __dadd_rn(__dmul_rn(sor2, fold), __ddiv_rn(__dmul_rn(t, sor1), cPP[k]));
-                res = __dadd_rn(res, fabs(__dsub_rn(fold, fnew)));
-                cur[k] = fnew;
-                sF[(s & 1) * nj + jj] = fnew;
-                fw = fnew;
+            const double *cf = sCf + (size_t)set * 6 * B * nj + jj;
+            const size_t cp = (size_t)B * nj;
+#pragma unroll
+            for (int u = 0; u < RELAX_BLOCK; ++u) {
+                const int s = s0 + u;
+                if (u >= B || s >= a.nstep) break;
+                if (u > 0) __syncthreads();
+                const int ii = s - jj;
+                if (rowthr && ii >= 0 && ii < ni) {
+                    const double *c = cf + (size_t)u * nj;
+                    const double fn = jj == nj - 1 ? sB[(set * 2 + 1) * B + u] : fnv[u];
+                    const double fe = ii == ni - 1 ? feast : fev[u];
+                    const double fs = jj == 0 ? sB[set * 2 * B + u] : sF[((s - 1) & 1) * nj + jj - 1];
+                    // FNEW = SOR2 FPZ + (RHSZ - ZN FN - ZS FS - ZE FE - ZW FW) SOR1 / PPP, rounded as written
+                    double t = __dsub_rn(c[CF_RHSZ * cp], __dmul_rn(c[CF_ZN * cp], fn));
+                    t = __dsub_rn(t, __dmul_rn(c[CF_ZS * cp], fs));
+                    t = __dsub_rn(t, __dmul_rn(c[CF_ZE * cp], fe));
+                    t = __dsub_rn(t, __dmul_rn(c[CF_ZW * cp], fw));
+                    const double fnew = __dadd_rn(__dmul_rn(sor2, fold), __ddiv_rn(__dmul_rn(t, sor1), c[CF_PPP * cp]));
+                    res = __dadd_rn(res, fabs(__dsub_rn(fold, fnew)));
+                    cur[(size_t)s * nj + jj] = fnew;
+                    sF[(s & 1) * nj + jj] = fnew;
+                    fw = fnew;
+                }
+                fold = fev[u];
             }
         }
+        asm volatile("cp.async.wait_all;" ::: "memory");
         if (dropped) return;
         if (rowthr) sRow[jj] = res;
         __syncthreads();

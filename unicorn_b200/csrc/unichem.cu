@@ -1615,8 +1615,10 @@ static int launch_relax(uc_ctx *ctx, cudaStream_t st, int nsm, RelaxBuffers &rb,
     // the bounded waits between passes give up after UNICHEM_RELAX_WAIT_NS nanoseconds of wall clock (2 s)
     a.timeout_ns = 2000000000LL;
     if (const char *e = getenv("UNICHEM_RELAX_WAIT_NS")) a.timeout_ns = std::max(0LL, atoll(e));
-    const int threads = (nj + 31) / 32 * 32;
-    const size_t smem = 3 * (size_t)nj * sizeof(double);
+    // a warp more than the rows need, where there is room, for the wait and the publication between passes
+    const int threads = std::min(RELAX_MAX_ROWS, (nj + 31) / 32 * 32 + 32);
+    const size_t smem = relax_smem(nj);
+    CK(cudaFuncSetAttribute(enth_relax_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, enth_relax_kernel, threads, smem));
     if (per_sm < 1) return set_err(ctx, UC_E_CUDA, "relaxation kernel does not fit on an SM");
