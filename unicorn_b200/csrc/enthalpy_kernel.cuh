@@ -5,7 +5,7 @@
 //   enth_source_kernel  heat release of the start-state rate coefficients and
 //                       the updated mass fractions: RA = RC * prod(Y), PRD,
 //                       PROD = sum PRD, QDSP, QDOT          (solveh.f:116-1145)
-//                       (two 16-warp CTAs per SM, RC read through L1)
+//                       (the rate kernel's generated species sums)
 //   enth_coef_kernel    EKT, EMU and the species-enthalpy diffusion factors
 //                       RDHSP_k of every cell      (spgsolv.f:174, solveh.f:39-57)
 //   enth_rhs_kernel     interior cells: coefficients ZE, ZW, ZN, ZS (hybrid
@@ -54,22 +54,20 @@ struct EnthSrcArgs {
     int npad, ntile;
 };
 
-constexpr size_t ENTH_SRC_SMEM = (size_t)(3 * LSP + 1) * TILE * sizeof(double);
+constexpr size_t ENTH_SRC_SMEM = (size_t)NPAIR * TILE * sizeof(double2) + (size_t)(3 * LSP + 2 * CHEM_WARPS) * TILE * sizeof(double);
 
-// RC is read straight from the plane (through L1: a row of the tile is read by
-// the PRD lists of several species), so that shared memory holds only the
-// tile's Y and the species sums and two CTAs share an SM: the loads of one
-// overlap the arithmetic of the other. (Staging the tile's RC block [544][32]
-// in shared memory allowed one CTA per SM: 2.98 ms for the C2 field, 3.7 % of
-// DRAM bandwidth, stalled on the barriers between its load and species phases.)
+// A tile's RC come to shared memory once, as the pairs the generated species sums of the rate kernel read, and
+// one CTA takes a tile at a time. Bound by those loads: 139 KB a tile, which with one CTA an SM do not overlap the
+// sums. Walking the PRD term lists in a table with RC from L1 took 1.0 ms on a 131 x 711 grid, this takes 0.26 ms
+// (1.7 TB/s of RC).
 template <typename RCT>
-__global__ void __launch_bounds__(CHEM_THREADS, 2) enth_source_kernel(const EnthSrcArgs a)
+__global__ void __launch_bounds__(CHEM_THREADS, 1) enth_source_kernel(const EnthSrcArgs a)
 {
     extern __shared__ __align__(16) double esm[];
-    double *sY = esm;                  // [52][32]
-    double *sP = sY + LSP * TILE;      // [52][32] PRD
-    double *sH = sP + LSP * TILE;      // [52][32] PRD * HENTH / HFO
-    double *sT = sH + LSP * TILE;      // [32] TKD
+    double2 *pr = reinterpret_cast<double2 *>(esm);   // [272][32] RC of a reaction and its reverse
+    double *sY = esm + 2 * NPAIR * TILE;              // [52][32]
+    double *sPL = sY + LSP * TILE;                    // [104][32] gain and loss sums
+    double *sR = sPL + 2 * LSP * TILE;                // [2][16][32] a warp's part of PROD and QDOT
     const DevParams &P = *a.P;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const size_t np = a.npad;
@@ -77,55 +75,47 @@ __global__ void __launch_bounds__(CHEM_THREADS, 2) enth_source_kernel(const Enth
         const size_t cell = (size_t)tile * TILE + lane;
         const bool f64 = sizeof(RCT) == 8 || (a.tile_flag && a.tile_flag[tile]);
         for (int k = warp; k < LSP; k += CHEM_WARPS) sY[k * TILE + lane] = a.y[(size_t)k * np + cell];
-        if (warp == 0) sT[lane] = a.tk[cell] * P.TSTR;
-        __syncthreads();
-        {
-            const double TKD = sT[lane];
-            const double TKD2 = TKD * TKD, TKD3 = TKD * TKD2, TKD4 = TKD * TKD3, TKD5 = TKD * TKD4;
-            const int ip = TKD > UC_TPOL1 ? 7 : 0;
-            const bool out = !(a.hold && a.hold[cell]);
-            const int ns = P.nspec_of_warp[warp];
-            for (int s = 0; s < ns; ++s) {
-                const int k = P.spec_of_warp[warp][s];
-                double prd = 0.0;
-                const int len = P.prd_len[k];
-                if (len > 0) {
-                    const int off = P.prd_off[k];
-                    double acc = 0.0;
-                    for (int t = 0; t < len; ++t) {
-                        const unsigned code = P.prd_term[off + t];
-                        const int r = code & 0x1FFF;
-                        double v = 0.0;
-                        if (!(code & 0x2000)) {           // SRA terms are zero (solveh.f:671-676)
-                            v = f64 ? __ldg(a.rc + (size_t)r * np + cell) : (double)__ldg(a.rc32 + (size_t)r * np + cell);
-                            for (int q = 0; q < P.ra_len[r]; ++q) v = v * sY[P.ra_sp[r * 3 + q] * TILE + lane];
-                            if (code & 0x4000) v = P.prd_coef[off + t] * v;
-                        }
-                        const bool neg = code & 0x8000;
-                        acc = (t == 0) ? (neg ? -v : v) : (neg ? acc - v : acc + v);
-                    }
-                    prd = P.WM[k] * P.HFO[k] * acc;
-                }
-                if (out) a.qdsp[(size_t)k * np + cell] = -(P.RCONV * prd / P.HFO[k]);
-                const double *pa = P.poly + k * 14 + ip;
-                const double HSSP = (pa[0] * TKD + pa[1] * TKD2 / 2.0 + pa[2] * TKD3 / 3.0 + pa[3] * TKD4 / 4.0 +
-                                     pa[4] * TKD5 / 5.0) / P.WM[k] * P.HCONVR;
-                const double H = HSSP * P.WMSTR * P.HSTR + pa[5] / P.WM[k] * P.GASC;
-                sP[k * TILE + lane] = prd;
-                sH[k * TILE + lane] = prd * H / P.HFO[k];
+        const double TKD = a.tk[cell] * P.TSTR;
+        if (f64) {
+#pragma unroll
+            for (int i = 0; i < NPAIR / CHEM_WARPS; ++i) {
+                const int p = warp + i * CHEM_WARPS;
+                const double *r = a.rc + (size_t)(2 * p) * np + cell;
+                pr[p * TILE + lane] = make_double2(__ldg(r), __ldg(r + np));
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < NPAIR / CHEM_WARPS; ++i) {
+                const int p = warp + i * CHEM_WARPS;
+                const float *r = a.rc32 + (size_t)(2 * p) * np + cell;
+                pr[p * TILE + lane] = make_double2((double)__ldg(r), (double)__ldg(r + np));
             }
         }
         __syncthreads();
-        if (warp == 0) {                      // ordered sums over the species (solveh.f:1134-1144)
-            double prod = 0.0, hrr = 0.0;
-            for (int k = 0; k < LSP; ++k) {
-                prod = prod + sP[k * TILE + lane];
-                hrr = hrr + sH[k * TILE + lane];
-            }
-            a.prod[cell] = prod;
-            if (!(a.hold && a.hold[cell])) a.qdot[cell] = -(hrr * P.RCONV);
-        }
+        tile_omega_sums(pr, sY, sPL, lane, warp);
         __syncthreads();
+        const bool out = !(a.hold && a.hold[cell]);
+        const double *hc = P.hc + (TKD > UC_TPOL1 ? 6 : 0);
+        double prod = 0.0, hrr = 0.0;
+        for (int k = warp; k < LSP; k += CHEM_WARPS) {
+            const double w = P.WM[k] * fma(-sY[k * TILE + lane], sPL[(LSP + k) * TILE + lane], sPL[k * TILE + lane]);
+            const double q = -(P.RCONV * w);
+            if (out) a.qdsp[(size_t)k * np + cell] = q;
+            const double *e = hc + k * 12;            // species enthalpy (solveh.f:39-57)
+            const double H = fma(TKD, fma(TKD, fma(TKD, fma(TKD, fma(TKD, e[4], e[3]), e[2]), e[1]), e[0]), e[5]);
+            prod = fma(w, P.HFO[k], prod);
+            hrr = fma(q, H, hrr);
+        }
+        sR[warp * TILE + lane] = prod;
+        sR[(CHEM_WARPS + warp) * TILE + lane] = hrr;
+        __syncthreads();
+        if (warp < 2) {                               // sums over the species (solveh.f:1134-1144)
+            double v = 0.0;
+            for (int i = 0; i < CHEM_WARPS; ++i) v = v + sR[(warp * CHEM_WARPS + i) * TILE + lane];
+            if (warp == 0) a.prod[cell] = v;
+            else if (out) a.qdot[cell] = v;
+        }
+        // the next tile's barriers order these reads before sR is written again
     }
 }
 
