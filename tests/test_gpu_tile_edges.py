@@ -116,3 +116,35 @@ def test_relaxation_at_block_edges(cuda, oracle, lj, li):
     fg, pg = cuda.enthalpy_relax(lj, li, g["rho"], o["rhsz"], o["z"], g["ht"], isor=5, tol=-1.0)
     assert pg == po
     assert np.array_equal(fg, fo)
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 129, 257])
+def test_surrogate_rows_do_not_depend_on_their_tile(cuda, n):
+    """The network's rows at the edges of the feature kernel's 32 cells and of the layers' 128-row tiles: the same
+    value bit for bit as in a field of 3,001 cells, where they stand in the middle (each row is its own sum)."""
+    from unicorn_b200.fields import batch_cells, nondimensional
+    from unicorn_b200.surrogate import Surrogate, raw_features
+    f = batch_cells(3001, seed=7)
+
+    def run(cells):
+        with cuda.UniChem(len(cells)) as u:
+            tk, rho = nondimensional(f, u.scales, u.wm)
+            u.upload(tk[cells], rho[cells], np.ascontiguousarray(f.y[:, cells]))
+            u.set_pressure(f.p[cells] / u.scales["PSTR"])
+            if not s.ready:
+                q = u.omega().qdsp
+                s.net.set_norm(**Surrogate.norm_from_sample(raw_features(f.T, f.p / (u.scales["PBACK"] * u.scales["PSTR"]), f.y), q))
+                s.ready = True
+            s.net.omega(u, tol=float("inf"))
+            out = {"qdsp": np.empty((52, len(cells)))}
+            u.download_outputs(out)
+        return out["qdsp"]
+
+    class s:
+        net, ready = Surrogate(capacity=4096, seed=3), False
+    try:
+        whole = run(np.arange(3001))
+        first = 1000
+        assert np.array_equal(run(np.arange(first, first + n)), whole[:, first:first + n])
+    finally:
+        s.net.close()

@@ -59,7 +59,7 @@ constexpr size_t ENTH_SRC_SMEM = (size_t)NPAIR * TILE * sizeof(double2) + (size_
 // A tile's RC come to shared memory once, as the pairs the generated species sums of the rate kernel read, and
 // one CTA takes a tile at a time. Bound by those loads: 139 KB a tile, which with one CTA an SM do not overlap the
 // sums. Walking the PRD term lists in a table with RC from L1 took 1.0 ms on a 131 x 711 grid, this takes 0.26 ms
-// (1.7 TB/s of RC).
+// (1.6 TB/s of RC).
 template <typename RCT>
 __global__ void __launch_bounds__(CHEM_THREADS, 1) enth_source_kernel(const EnthSrcArgs a)
 {

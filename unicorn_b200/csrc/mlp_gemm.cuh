@@ -316,20 +316,26 @@ namespace uc {
 // One layer of the network over many rows, weights resident in shared memory:
 //   out[M, N] = epi(A[M, K] * W[N, K]^T + bias),   N in {64, 128, 192, 256}, K in {64, 128, 192, 256}
 // A persistent CTA per SM, warp-specialised:
-//   warp 8 (one thread): TMA loads. W once (K/64 boxes of N rows x 128 B), then
+//   warp 16 (one thread): TMA loads. W once (K/64 boxes of N rows x 128 B), then
 //     the 128 x 64 chunks of the CTA's row tiles, in order, into a ring of
 //     LW_SLOTS 16 KB slots; a slot is refilled once the MMAs that read it have
 //     completed (their commit arrives on the slot's "empty" barrier);
-//   warp 9 (one thread): for each tile, once the epilogue has drained the
+//   warp 17 (one thread): for each tile, once the epilogue has drained the
 //     accumulator it is about to use (two accumulators of 256 TMEM columns),
 //     four tcgen05.mma (K = 16) per chunk as each chunk lands, a commit per
 //     chunk (frees the slot) and one per tile (the accumulator is full);
-//   warps 0-7: drain the full accumulator through tcgen05.ld, 32 columns at a
+//   warps 0-15: drain the full accumulator through tcgen05.ld, 32 columns at a
 //     time, into the epilogue (bias from shared
 //     memory, then GELU -> BF16 with the pre-activation kept if asked, bias ->
 //     FP32, or the surrogate's decoding into FP64 omega; 16-byte stores) and
-//     mark it empty. Warp w reads TMEM lanes 32 (w % 4) .. +31 and half w / 4
-//     of the columns.
+//     mark it empty. Warp w reads TMEM lanes 32 (w % 4) .. +31 and every
+//     fourth block of 32 columns from w / 4 on.
+// The epilogue bounds the layer where it is not HBM (512 MB for 500,001 rows
+// of 256: 77 us at the measured copy rate). A thread holds a row, so its BF16
+// stores straight from registers spread each store instruction over 32 lines
+// (137 us a layer, with eight epilogue warps); the warp's 32 x 32 block goes
+// through shared memory instead, and a store instruction covers 8 lines with
+// whole sectors: LW_NOTE.
 // So the loads of the next tiles, the MMAs of this one and the epilogue of the
 // previous one overlap. Operands are in the 128-byte-swizzled K-major layout
 // that TMA writes with CU_TENSOR_MAP_SWIZZLE_128B (rows of 64 BF16, 16-byte
@@ -337,12 +343,15 @@ namespace uc {
 // is bounded; a wait that gives up sets the status and an abort flag that the
 // other roles see, and the CTA retires its copies and MMAs in flight before it
 // frees TMEM.
-constexpr int LW_EPI_WARPS = 8;
+constexpr int LW_EPI_WARPS = 16;
 constexpr int LW_THREADS = (LW_EPI_WARPS + 2) * 32;
-constexpr int LW_SLOTS = 5;                                    // A chunks in flight per CTA
+constexpr int LW_SLOTS = 4;                                    // A chunks in flight per CTA
 constexpr uint32_t LW_CHUNK_BYTES = (uint32_t)GM * GK * 2;     // 128 rows x 64 BF16
 constexpr size_t LW_W_BYTES = (size_t)256 * 256 * 2;
-constexpr size_t LW_SMEM = 1024 + LW_W_BYTES + (size_t)LW_SLOTS * LW_CHUNK_BYTES + 256;   // align slack, W, ring, barriers
+constexpr uint32_t LW_STAGE_BYTES = 32 * 32 * 2;               // a warp's 32 rows x 32 BF16
+constexpr int LW_BARS = 2 * LW_SLOTS + 6;
+// align slack, W, ring, the epilogue warps' staging
+constexpr size_t LW_SMEM = 1024 + LW_W_BYTES + (size_t)LW_SLOTS * LW_CHUNK_BYTES + (size_t)LW_EPI_WARPS * LW_STAGE_BYTES;
 
 // 32 consecutive TMEM columns of the warp's 32 lanes into v (asynchronous until tm_wait32(v))
 __device__ __forceinline__ void tm_ld32(uint32_t (&v)[32], uint32_t taddr)
@@ -377,13 +386,13 @@ __device__ __forceinline__ double lw_decode(float t, float scale)
     return (double)scale * (double)(at < 0.25f ? small : big);
 }
 
-// epilogue of 32 accumulator columns [c, c + 32) of one row (bias read as float4 broadcasts)
-__device__ __forceinline__ void lw_store32(const GemmArgs &g, const uint32_t (&v)[32], int row, int c,
-                                           const float *s_bias, const float (*s_dec)[64])
+// epilogue of 32 accumulator columns [c, c + 32) of the warp's 32 rows, one a lane (bias read as float4 broadcasts)
+__device__ __forceinline__ void lw_store32(const GemmArgs &g, const uint32_t (&v)[32], int row, int c, int lane,
+                                           const float *s_bias, const float (*s_dec)[64], unsigned char *stage)
 {
-    if (row >= g.M) return;
     const float4 *b4 = reinterpret_cast<const float4 *>(s_bias + c);
     if (g.epi == EPI_BIAS_GELU) {
+        __syncwarp();                  // the block before has been read
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             __align__(16) __nv_bfloat162 o[4];
@@ -393,7 +402,7 @@ __device__ __forceinline__ void lw_store32(const GemmArgs &g, const uint32_t (&v
                 const int i = q * 8 + j * 4;
                 const float z0 = __uint_as_float(v[i]) + bb.x, z1 = __uint_as_float(v[i + 1]) + bb.y;
                 const float z2 = __uint_as_float(v[i + 2]) + bb.z, z3 = __uint_as_float(v[i + 3]) + bb.w;
-                if (g.z_save) {
+                if (g.z_save && row < g.M) {
                     float4 zz;
                     zz.x = z0; zz.y = z1; zz.z = z2; zz.w = z3;
                     *reinterpret_cast<float4 *>(g.z_save + (size_t)row * g.ldz + c + i) = zz;
@@ -401,12 +410,24 @@ __device__ __forceinline__ void lw_store32(const GemmArgs &g, const uint32_t (&v
                 o[j * 2] = __floats2bfloat162_rn(gelu_f(z0), gelu_f(z1));
                 o[j * 2 + 1] = __floats2bfloat162_rn(gelu_f(z2), gelu_f(z3));
             }
-            *reinterpret_cast<uint4 *>(g.out_bf16 + (size_t)row * g.ldo + c + q * 8) = *reinterpret_cast<uint4 *>(o);
+            // 16-byte piece q of the lane's row, at a place that keeps both directions free of bank conflicts
+            *reinterpret_cast<uint4 *>(stage + lane * 64 + ((q ^ ((lane >> 1) & 3)) * 16)) = *reinterpret_cast<uint4 *>(o);
         }
-    } else if (g.epi == EPI_DECODE) {
-        // straight into the [k][ld] FP64 output: the lanes are consecutive rows
+        __syncwarp();
+        const int r0 = row - lane, p = lane & 3;
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
+        for (int i = 0; i < 4; ++i) {
+            const int r = i * 8 + (lane >> 2);
+            const uint4 o = *reinterpret_cast<const uint4 *>(stage + r * 64 + ((p ^ ((r >> 1) & 3)) * 16));
+            if (r0 + r < g.M) *reinterpret_cast<uint4 *>(g.out_bf16 + (size_t)(r0 + r) * g.ldo + c + p * 8) = o;
+        }
+        return;
+    }
+    if (row >= g.M) return;
+    if (g.epi == EPI_DECODE) {
+        // straight into the [k][ld] FP64 output, 16 columns a warp: the lanes are consecutive rows
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
             const int k = c + j;
             if (k < g.dec_n) {
                 const float t = fmaf(__uint_as_float(v[j]), s_dec[0][k], s_dec[1][k]);
@@ -431,13 +452,15 @@ __global__ void __launch_bounds__(LW_THREADS, 1)
     gemm_w_resident_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
                            const __grid_constant__ CUtensorMap map_w)
 {
-    extern __shared__ __align__(1024) unsigned char lsm_raw[];
+    extern __shared__ __align__(16) unsigned char lsm_raw[];
     // 1024-byte alignment of the swizzle atoms, whatever the base of dynamic shared memory
     unsigned char *lsm = lsm_raw + ((1024 - (smem_u32(lsm_raw) & 1023)) & 1023);
     const int N = g.N, K = g.K, nck = K / GK;
     unsigned char *sW = lsm;                                           // K/64 chunks of N x 128 B
     unsigned char *sA = lsm + LW_W_BYTES;                              // LW_SLOTS chunks of 128 x 128 B
-    uint64_t *full = reinterpret_cast<uint64_t *>(sA + (size_t)LW_SLOTS * LW_CHUNK_BYTES);
+    unsigned char *sStage = sA + (size_t)LW_SLOTS * LW_CHUNK_BYTES;    // a block per epilogue warp
+    __shared__ uint64_t s_bars[LW_BARS];
+    uint64_t *full = s_bars;
     uint64_t *empty = full + LW_SLOTS;
     uint64_t *accf = empty + LW_SLOTS;       // [2] accumulator full (MMA commit)
     uint64_t *acce = accf + 2;               // [2] accumulator drained (one arrive per epilogue warp)
@@ -447,6 +470,7 @@ __global__ void __launch_bounds__(LW_THREADS, 1)
     __shared__ __align__(16) float s_bias[256];
     __shared__ float s_dec[3][64];           // EPI_DECODE: t = acc * sd + (bias * sd + mu), scale
     __shared__ volatile int s_abort;
+    static_assert(LW_SMEM + 2048 <= 232448, "shared memory of an SM");
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int ntiles = (g.M + GM - 1) / GM;
 
@@ -543,9 +567,8 @@ __global__ void __launch_bounds__(LW_THREADS, 1)
             mbar_wait_bounded(done, 0, 1 << 22);         // no MMA in flight when TMEM is freed
         }
     } else {
-        // ---- epilogue warps: warp w drains TMEM lanes 32 (w % 4) .. +31 (rows), columns [w / 4 * N / 2, +N / 2),
-        // 32 at a time
-        const int ncw = N / 2, cbeg = (warp >> 2) * ncw;
+        // ---- epilogue warps: warp w drains TMEM lanes 32 (w % 4) .. +31 (rows), every fourth block of 32 columns
+        unsigned char *stage = sStage + (size_t)warp * LW_STAGE_BYTES;
         int it = 0;
         for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
             const int b = it & 1;
@@ -553,11 +576,13 @@ __global__ void __launch_bounds__(LW_THREADS, 1)
             tc_fence_after();
             const int row = tile * GM + (warp & 3) * 32 + lane;
             const uint32_t tbase = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(b * 256);
-            for (int c = cbeg; c < cbeg + ncw; c += 32) {
+            // (the decoding output layer has 64 columns at most: 16 for each of the four warps of a row)
+            const int cw = g.epi == EPI_DECODE ? 16 : 32;
+            for (int c = (warp >> 2) * cw; c < N; c += LW_EPI_WARPS / 4 * cw) {
                 uint32_t v[32];
                 tm_ld32(v, tbase + (uint32_t)c);
                 tm_wait32(v);
-                lw_store32(g, v, row, c, s_bias, s_dec);
+                lw_store32(g, v, row, c, lane, s_bias, s_dec, stage);
             }
             tc_fence_before();
             __syncwarp();
