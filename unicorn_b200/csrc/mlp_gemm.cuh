@@ -335,7 +335,8 @@ namespace uc {
 // stores straight from registers spread each store instruction over 32 lines
 // (137 us a layer, with eight epilogue warps); the warp's 32 x 32 block goes
 // through shared memory instead, and a store instruction covers 8 lines with
-// whole sectors: LW_NOTE.
+// whole sectors (101 us). The decoding output layer, 16 columns a warp on all
+// sixteen, takes 109 us (177 with 32 columns on eight of them).
 // So the loads of the next tiles, the MMAs of this one and the epilogue of the
 // previous one overlap. Operands are in the 128-byte-swizzled K-major layout
 // that TMA writes with CU_TENSOR_MAP_SWIZZLE_128B (rows of 64 BF16, 16-byte
