@@ -76,8 +76,9 @@ __global__ void __launch_bounds__(PROP_THREADS, 4) props_fp64_kernel(const PropA
         for (int j = warp; j < nc; j += PROP_THREADS / 32) {
             const double y0 = sY[lane][j];
             const double y1 = two && lane + 32 < LSP - 1 ? sY[k1][j] : 0.0;
-            // sub-mixture: species with Y >= 1e-3 plus N2 (main:842-915)
-            const bool in0 = y0 >= 1.0e-03, in1 = y1 >= 1.0e-03, isn2 = lane + 32 == LSP - 1;
+            // sub-mixture: all species but those with Y < 1e-3 (a NaN stays in and shows in the results), plus N2
+            // (main:842-915)
+            const bool in0 = !(y0 < 1.0e-03), in1 = !(y1 < 1.0e-03), isn2 = lane + 32 == LSP - 1;
             const double iw0 = P.tbw[lane], iw1 = P.tbw[k1];
             double x0 = in0 ? y0 * iw0 : 0.0, x1 = in1 ? y1 * iw1 : 0.0;
             double mass = (in0 ? y0 : 0.0) + (in1 ? y1 : 0.0), TMOLE = x0 + x1;
