@@ -52,7 +52,6 @@ struct uc_ctx {
     // fields of up to STAGE_CELLS cells: pinned staging of the host copies (upload rows, then download rows and
     // the status word), read and written by one kernel each; null for larger fields
     double *stage = nullptr;
-    cudaEvent_t stage_read = nullptr;  // the last upload kernel has read its rows
     uc_scales sc{};
     uc_inputs inputs{};               // the input-card values of uc_init
     DevParams *hP = nullptr;          // host copy
@@ -486,7 +485,6 @@ static void free_ctx(uc_ctx *c)
     for (auto e : c->ev_pool) cudaEventDestroy(e);
     c->ev_pool.clear();
     if (c->stage) cudaFreeHost(c->stage);
-    if (c->stage_read) cudaEventDestroy(c->stage_read);
     if (c->stream) cudaStreamDestroy(c->stream);
     if (c->io_stream) cudaStreamDestroy(c->io_stream);
     if (c->io_event) cudaEventDestroy(c->io_event);
@@ -559,9 +557,9 @@ static int check_status(uc_ctx *ctx)
 
 // Host copies of a small field. A pageable copy costs 8-10 us whatever its size, and an upload has eleven copies,
 // fills and pad launches, a download up to four copies and a wait: for a few hundred cells those calls were
-// most of the time (one cell, upload and omega: 131 us, of which 28 the rate kernel; 62 us this way). Up to STAGE_CELLS cells the host rows
-// go through pinned memory that one kernel reads or writes in place; beyond, the copies' bandwidth decides and
-// they stay.
+// most of the time (one cell, upload and omega: 131 us, of which 28 the rate kernel; 73 us this way, 10 of them the
+// upload's wait). Up to STAGE_CELLS cells the host rows go through pinned memory that one kernel reads or writes in
+// place; beyond, the copies' bandwidth decides and they stay.
 constexpr int STAGE_CELLS = 512;
 constexpr int STAGE_UP = LSP + 4, STAGE_DOWN = 3 * LSP + 5;       // rows: tk, rho, Y, soot; the most a call returns
 
@@ -742,9 +740,8 @@ extern "C" int uc_init(const uc_inputs *in, int ncell, int device, uc_ctx **out)
             break;
         cudaMemset(ctx->sour, 0, 6 * np * sizeof(double));
         if (ncell <= STAGE_CELLS &&
-            (cudaEventCreateWithFlags(&ctx->stage_read, cudaEventDisableTiming) != cudaSuccess ||
-             cudaHostAlloc((void **)&ctx->stage, ((size_t)(STAGE_UP + STAGE_DOWN) * ncell + 1) * sizeof(double),
-                           cudaHostAllocDefault) != cudaSuccess)) {
+            cudaHostAlloc((void **)&ctx->stage, ((size_t)(STAGE_UP + STAGE_DOWN) * ncell + 1) * sizeof(double),
+                          cudaHostAllocDefault) != cudaSuccess) {
             ctx->stage = nullptr;             // without it the copies of larger fields serve
             cudaGetLastError();
         }
@@ -834,7 +831,6 @@ extern "C" int uc_upload_fields(uc_ctx *ctx, const double *tk, const double *rho
     if (!ctx || !tk || !rho || !fsp) return set_err(ctx, UC_E_ARG, "uc_upload_fields: tk, rho and fsp are required");
     CK(cudaSetDevice(ctx->device));
     if (ctx->stage) {
-        CK(cudaEventSynchronize(ctx->stage_read));      // the last upload has left the staging rows
         const size_t row = (size_t)ctx->n * sizeof(double);
         double *s = ctx->stage;
         memcpy(s, tk, row);
@@ -849,7 +845,8 @@ extern "C" int uc_upload_fields(uc_ctx *ctx, const double *tk, const double *rho
         stage_upload_kernel<<<std::min((STAGE_UP * ctx->npad + 255) / 256, 2 * ctx->nsm), 256, 0, ctx->stream>>>(
             ctx->stage, ctx->n, ctx->npad, ctx->tk, ctx->rho, ctx->y, ctx->y0, ctx->soot, ctx->soot0);
         CK(cudaGetLastError());
-        CK(cudaEventRecord(ctx->stage_read, ctx->stream));
+        // complete on return, as with the copies: the staging rows are free, and other streams may read the fields
+        CK(cudaStreamSynchronize(ctx->stream));
         ctx->have_fields = true;
         ctx->have_rc = false;
         ctx->rc_start = false;
