@@ -330,6 +330,16 @@ __host__ __device__ constexpr size_t relax_smem(int nj)
 {
     return sizeof(double) * (3 * (size_t)nj + 2 * (size_t)relax_block(nj) * (6 * (size_t)nj + 2));
 }
+// the most that any number of rows needs (916 rows: 198 KB): what the kernel is allowed on every device, once and for
+// all grids, since the allowance belongs to the function and threads with other grids launch it too
+constexpr size_t relax_smem_max()
+{
+    size_t m = 0;
+    for (int nj = 1; nj <= RELAX_MAX_ROWS; ++nj) m = relax_smem(nj) > m ? relax_smem(nj) : m;
+    return m;
+}
+constexpr size_t RELAX_SMEM_MAX = relax_smem_max();
+static_assert(RELAX_SMEM_MAX + 1024 <= 232448, "shared memory of the relaxation");
 
 __device__ __forceinline__ void cp_async8(double *dst, const double *src)
 {

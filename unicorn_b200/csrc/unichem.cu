@@ -1615,7 +1615,7 @@ static int launch_relax(uc_ctx *ctx, cudaStream_t st, int nsm, RelaxBuffers &rb,
     // a warp more than the rows need, where there is room, for the wait and the publication between passes
     const int threads = std::min(RELAX_MAX_ROWS, (nj + 31) / 32 * 32 + 32);
     const size_t smem = relax_smem(nj);
-    CK(cudaFuncSetAttribute(enth_relax_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CK(cudaFuncSetAttribute(enth_relax_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RELAX_SMEM_MAX));
     int per_sm = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, enth_relax_kernel, threads, smem));
     if (per_sm < 1) return set_err(ctx, UC_E_CUDA, "relaxation kernel does not fit on an SM");
