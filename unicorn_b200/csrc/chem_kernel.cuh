@@ -74,14 +74,6 @@ __device__ __forceinline__ void tile_scalars(const DevParams &P, double *sC, int
     sC[SC_STND * TILE + lane] = stnd;
 }
 
-// x / T with 1 / T at hand: the quotient corrected by its residual (as exact as the division but for the last
-// bit in rare cases), for the exponents, where an error is multiplied by the exponent's size.
-__device__ __forceinline__ double over_t(double x, double TKD, double IT)
-{
-    const double q = CO_MUL(x, IT);
-    return CO_FMA(CO_FMA(-q, TKD, x), IT, q);
-}
-
 // The soot sources (ckrates.f:1337-1352).
 __device__ __forceinline__ void soot_sources(const DevParams &P, const double *sC, double *sour, size_t sstride,
                                              size_t soff, int lane)

@@ -133,20 +133,6 @@ __device__ __forceinline__ void co_sync(const CoTile &c) { asm volatile("bar.syn
 #define CO_WAIT_P(set) asm volatile("bar.sync %0, 96;" ::"r"(c.id + 2 + (set)))
 #define CO_ARRIVE_P(set) asm volatile("bar.arrive %0, 96;" ::"r"(c.id + 2 + (set)))
 
-// n / d without the branch of the compiler's division, which would end the scheduling of the statements around
-// it and is three times the instructions: the hardware's reciprocal approximation r, one step of third order for
-// the quotient (with e = 1 - d r, 1 / d = r (1 + e + e^2 + ...)), and the residual correction of Markstein (IBM J.
-// Res. Dev. 34, 1990), which leaves at most the last bit in doubt. Where the residual is no number (an operand or the
-// quotient infinite, or d zero or below the normal range), n r is IEEE's result.
-__device__ __forceinline__ double co_quot(double n, double d)
-{
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-    const double e = __fma_rn(-d, r, 1.0), q0 = __dmul_rn(n, r);
-    const double q = __fma_rn(q0, __fma_rn(e, e, e), q0), m = __fma_rn(-d, q, n);
-    return m == m ? __fma_rn(m, r, q) : q0;
-}
-
 __device__ __forceinline__ void co_st2(double *p, double a, double b)
 {
     asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(smem_u32(p)), "d"(a), "d"(b));
