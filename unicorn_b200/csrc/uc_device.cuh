@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "generated/mech_tables.h"
+#include "rate_limits.h"
 
 namespace uc {
 
@@ -11,7 +12,7 @@ constexpr int LSP = UC_LSP;
 constexpr int LRX = UC_LRX;
 constexpr int NPAIR = UC_NPAIR;
 constexpr int TILE = 32;                 // cells per tile = lanes of a warp
-constexpr int CHEM_WARPS = 16;           // warps of the rate/omega kernel
+constexpr int CHEM_WARPS = RATE_WARPS;   // warps of the rate/omega kernel
 constexpr int CHEM_THREADS = CHEM_WARPS * 32;
 constexpr int MAX_SPEC_PER_WARP = 8;
 constexpr int PROP_ROWS = 24;            // see DevParams::prow
@@ -43,7 +44,7 @@ struct PairSrc {
 // scalar rows (SC_*, 0: none) of the tile, so nothing is decoded or divided per cell.
 struct __align__(16) PairTab {
     double akf, alf, exaf, c0, c1, pad0;
-    uint8_t g[6], ng, rut;                 // rows of the G table (k: G_k, 52 + k: 1 / G_k); ng = 0: no reverse
+    uint8_t g[KC_MAX], ng, rut;            // rows of the G table (k: G_k, 52 + k: 1 / G_k); ng = 0: no reverse
     uint8_t r0, t0, r1, t1;                // rows of rho^order (0: the slot is never written) and of the third body
     uint8_t y0, y1, fall, pad1;            // species whose Y is a factor (255: none); 1 + fall-off entry (0: none)
 };
@@ -53,9 +54,8 @@ struct __align__(16) FallTab {
     int dmole, pad;                        // scalar row of the third body
 };
 static_assert(sizeof(FallTab) == 64, "FallTab layout");
-constexpr int NFALL = 24;                  // entries of the fall-off table (the mechanism has 21)
 // both tables lie one after the other, staged into shared memory by bulk (TMA) copies at kernel start
-constexpr int PAIRTAB_BYTES = NPAIR * (int)sizeof(PairTab) + NFALL * (int)sizeof(FallTab);
+constexpr int PAIRTAB_BYTES = NPAIR * (int)sizeof(PairTab) + FALL_MAX * (int)sizeof(FallTab);
 static_assert(PAIRTAB_BYTES % 16 == 0, "bulk copy size must be a multiple of 16 bytes");
 
 // Constants of one context: scales, tables prepared at set-up, and the
@@ -99,7 +99,7 @@ struct DevParams {
     int8_t spec_of_warp[CHEM_WARPS][MAX_SPEC_PER_WARP];
     int8_t nspec_of_warp[CHEM_WARPS];
     // reaction pairs assigned to each warp (balanced by cost)
-    int16_t pair_of_warp[CHEM_WARPS][24];
+    int16_t pair_of_warp[CHEM_WARPS][WARP_ITEMS];
     int8_t npair_of_warp[CHEM_WARPS];
     int soot_warp;                        // the warp (of 16) that forms the soot sources
 };

@@ -366,7 +366,7 @@ static void build_params(const uc_inputs &in, DevParams &P, std::vector<uint8_t>
         };
         assemble(T.rc_order0, T.rc_tb0, T.rc_len0, T.rc_kind0, T.rc_idx0, D.c0, D.r0, D.t0, D.y0);
         assemble(T.rc_order1, T.rc_tb1, T.rc_len1, T.rc_kind1, T.rc_idx1, D.c1, D.r1, D.t1, D.y1);
-        if (T.aklow != 0.0 && nf < NFALL) {
+        if (T.aklow != 0.0) {              // (UC_FALLOFF of them)
             FallTab &F = ft[nf];
             F.aklow = T.aklow; F.allow = T.allow; F.ealow = T.ealow;
             for (int c = 0; c < 4; ++c) F.troe[c] = T.troe[c];
@@ -430,11 +430,11 @@ static void build_params(const uc_inputs &in, DevParams &P, std::vector<uint8_t>
     }
     std::vector<std::vector<int>> pw, sw;
     pcost.push_back(60.0);             // the soot sources, as one more item
-    balance(pcost, CHEM_WARPS, 25, pw);
+    balance(pcost, CHEM_WARPS, WARP_ITEMS, pw);
     for (int w = 0; w < CHEM_WARPS; ++w)
         for (int p : pw[w]) {
             if (p == NPAIR) P.soot_warp = w;
-            else if (P.npair_of_warp[w] < 24) P.pair_of_warp[w][P.npair_of_warp[w]++] = (int16_t)p;
+            else P.pair_of_warp[w][P.npair_of_warp[w]++] = (int16_t)p;
         }
     std::vector<double> scost(LSP);
     for (int k = 0; k < LSP; ++k) scost[k] = 8.0 + 2.0 * uc_prd_len[k] + 2.5 * uc_loss_len[k];

@@ -1153,6 +1153,9 @@ def gen_tables(mech: dict) -> str:
             rev_sp[r0 * QMAX + t] = sp - 1
             rev_div[r0 * QMAX + t] = 1 if op == "/" else 0
     out.append(f"#define UC_QMAX {QMAX}")
+    out.append(f"#define UC_QMIN {min(len(v['q']) for v in mech['reverse'].values())}")
+    # fall-off pairs: a negative AKF of the forward slot marks them (src/unicornd-mild-sd-5.f:364-413)
+    out.append(f"#define UC_FALLOFF {sum(x['akf'] < 0 and x['aklow'] != 0 for x in R[::2])}")
     out.append(arr("uc_rev_has", "int8_t", map(str, rev_has), 32))
     out.append(arr("uc_rev_rut", "int8_t", map(str, rev_rut), 32))
     out.append(arr("uc_rev_len", "int8_t", map(str, rev_len), 32))
@@ -1170,6 +1173,7 @@ def gen_tables(mech: dict) -> str:
             tsg.append(s)
             tco.append(0.0 if c is None else c)
             thc.append(0 if c is None else 1)
+    out.append(f"#define UC_NTB {len(mech['tb']) - 1}")
     out.append(arr("uc_tb_off", "int16_t", map(str, tbo), 16))
     out.append(arr("uc_tb_len", "int16_t", map(str, tbn), 16))
     out.append(arr("uc_tb_sp", "int8_t", map(str, tsp), 32))
@@ -1194,6 +1198,7 @@ def gen_tables(mech: dict) -> str:
             rc_kind[r0 * PMAX + t] = 1 if kind == "Y" else 0   # 1: *Y_idx, 0: /W_idx
             rc_idx[r0 * PMAX + t] = idx - 1
     out.append(f"#define UC_PMAX {PMAX}")
+    out.append(f"#define UC_RC_YMAX {max(sum(kind == 'Y' for _, kind, _ in v['post']) for v in mech['rc'].values())}")
     out.append(arr("uc_rc_order", "int8_t", map(str, rc_order), 32))
     out.append(arr("uc_rc_tb", "int8_t", map(str, rc_tb), 32))
     out.append(arr("uc_rc_len", "int8_t", map(str, rc_len), 32))
