@@ -219,7 +219,8 @@ __device__ __forceinline__ void tile_rates_fp64(const DevParams &P, const PairTa
             double kf = CO_MUL(T.akf, exp(CO_FMA(T.alf, ELOGT, -over_t(T.exaf, TKD, IT))));
             double kr = 0.0;
             if (T.ng) {
-                // 1/q, the factors of q and of its divisor in turn
+                // 1/q, the factors of q and of its divisor in turn (every partial product is a normal number from 138 K
+                // on; below 120 K the quotient in the source's order is none for other pairs)
                 double iq = CO_MUL(CO_MUL(sG[T.g[0] * TILE + lane], sG[T.g[1] * TILE + lane]), sG[T.g[2] * TILE + lane]);
                 for (int t = 3; t < T.ng; ++t) iq = CO_MUL(iq, sG[T.g[t] * TILE + lane]);
                 kr = T.rut ? CO_MUL(CO_MUL(kf, sC[T.rut * TILE + lane]), iq) : CO_MUL(kf, iq);

@@ -1,5 +1,6 @@
 // Generated by unicorn_b200/mech/codegen.py: the in-place species-update program
 // (src/lib/solvesp.f:85-2806) for a tile whose RC block is held on chip.
+// Run by the host test of the generated programs; the kernels run update_program_co.cuh.
 // RC slots 0..255 in tensor memory (slot i in columns 2i, 2i+1: low and high
 // word), slots 256..543 in shared memory. Requires RCS(i) (shared-memory row i of the
 // cell), TM_LD(bank, q, col) (load the double at column col into slot q of a

@@ -266,8 +266,8 @@ __global__ void temperature_held_kernel(const DevParams *Pp, const double *enth,
 
 // ---- stable counting sort of positions by n_sub, largest first.
 // Chunk j of `chunk` cells is owned by CTA j; key = nsub_max - n_sub. A chunk is scattered by one warp, 32 cells
-// after 32 (67 us for 4096 cells, 14 us for 512), so small fields have small chunks; up to 256 of them, which one CTA scans.
-// The order does not depend on the chunks.
+// after 32 (67 us for 4096 cells, 14 us for 512), so small fields have small chunks: up to 256 of them to 1,048,576
+// cells, beyond that more of 4096; one CTA scans their counts. The order does not depend on the chunks.
 __host__ __device__ constexpr int sort_chunk(int n) { return n <= 256 * 512 ? 512 : n <= 256 * 2048 ? 2048 : 4096; }
 constexpr int SORT_MAXBIN = 1024;
 

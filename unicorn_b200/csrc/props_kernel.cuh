@@ -1,6 +1,6 @@
-// Property kernels: Y clip + mixture-averaged transport, cp/h (FP64, or with the
-// property arithmetic in FP32 for the mixed form), and temperature from
-// enthalpy (FP64). Thread = cell.
+// Property kernels: Y clip + mixture-averaged transport (FP64: a warp takes a cell; mixed
+// form, with the pair terms in FP32: a thread takes one), cp/h (FP64: a thread takes a cell,
+// or in small fields a block 32 cells) and temperature from enthalpy (FP64, a thread a cell).
 #pragma once
 #include "uc_device.cuh"
 
@@ -30,6 +30,8 @@ __device__ __forceinline__ int ci_range(double TKDS)
 // and D_k goes out through shared memory, in rows of cells. The divisions and square roots of each pair are
 // divisions and square roots of each species: X_b / D_kb is X_b CI / (WMCD TKBP) from a table of
 // reciprocals, sqrt(ATC_k / ATC_b) a product of the two species' roots.
+//
+// The roots are taken per species, so ATC and AMU have to be positive: the fits give that from 20 to 6,000 K.
 //
 // What bounds it: FP64 latency (a cell is one chain of sums; four blocks per SM hide part of it). A thread per
 // cell, as before (a chain of about 300 pairs per thread, its lists in local memory), took 150 us for

@@ -557,9 +557,10 @@ static int check_status(uc_ctx *ctx)
 
 // Host copies of a small field. A pageable copy costs 8-10 us whatever its size, and an upload has eleven copies,
 // fills and pad launches, a download up to four copies and a wait: for a few hundred cells those calls were
-// most of the time (one cell, upload and omega: 131 us, of which 28 the rate kernel; 73 us this way, 10 of them the
-// upload's wait). Up to STAGE_CELLS cells the host rows go through pinned memory that one kernel reads or writes in
-// place; beyond, the copies' bandwidth decides and they stay.
+// most of the time. Up to STAGE_CELLS cells the host rows go through pinned memory that one kernel reads or writes in
+// place; beyond, they are copied. Upload and omega of 1, 512, 1,024, 2,048 and 4,096 cells took 126, 167, 207, 296 and
+// 465 us with copies and 70, 110, 168, 283 and 503 us staged (the rate kernel 48 us of each). They meet near 2,500 cells;
+// at 512 staging is a third ahead and a context's pinned rows are 0.9 MB.
 constexpr int STAGE_CELLS = 512;
 constexpr int STAGE_UP = LSP + 4, STAGE_DOWN = 3 * LSP + 5;       // rows: tk, rho, Y, soot; the most a call returns
 

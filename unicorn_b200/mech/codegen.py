@@ -291,7 +291,8 @@ def gen_tr_program(blocks, uses: dict, shadow: list[int]) -> str:
     between two register banks: the loads of segment s+1 are issued before the
     statements of segment s run and waited for after them, so their latency is
     hidden behind segment s. The arithmetic, its operands and their order are
-    those of the in-place program."""
+    those of the in-place program. The kernels run the grouped form below (gen_co_program); this one, whose
+    arithmetic is the two-array program's bit for bit, is run by the host test of the generated programs."""
     import re
     ctx = _TRCtx(uses)
     body = [f"UC_TR_PF(0, {blocks[0]['species']});"]
@@ -368,6 +369,7 @@ def gen_tr_program(blocks, uses: dict, shadow: list[int]) -> str:
         16 * len(blocks) + 19
     L = ["// Generated by unicorn_b200/mech/codegen.py: the in-place species-update program",
          "// (src/lib/solvesp.f:85-2806) for a tile whose RC block is held on chip.",
+         "// Run by the host test of the generated programs; the kernels run update_program_co.cuh.",
          f"// RC slots 0..{len(trow) - 1} in tensor memory (slot i in columns 2i, 2i+1: low and high",
          f"// word), slots {len(trow)}..{LRX - 1} in shared memory. Requires RCS(i) (shared-memory row i of the",
          "// cell), TM_LD(bank, q, col) (load the double at column col into slot q of a",
@@ -438,10 +440,6 @@ def _grouped_sums(blocks):
             d.append(ts)
         out.append(d)
     return out
-
-
-def _pair(t):
-    return t[1][1] // 2 if t[1] is not None and t[1][0] == "RC" else -1
 
 
 def _runs(sums):
@@ -1272,7 +1270,8 @@ def main():
     (GEN / "update_program_tr.cuh").write_text(gen_tr_program(blocks, uses, gen_inplace_program.shadow))
     (GEN / "update_program_co.cuh").write_text(gen_co_program(blocks))
     (GEN / "omega_program.cuh").write_text(gen_omega_program(mech))
-    print(f"wrote {GEN / 'mech_tables.h'}, {GEN / 'update_program.cuh'} and {GEN / 'update_program_tr.cuh'}")
+    print("wrote", ", ".join(str(GEN / f) for f in ("mech_tables.h", "update_program.cuh", "update_program_tr.cuh",
+                                                   "update_program_co.cuh", "omega_program.cuh")))
 
 
 if __name__ == "__main__":
