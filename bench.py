@@ -260,8 +260,8 @@ def fp64_fma_peak(dev):
 
 
 # DRAM read + write of one launch of the tile-resident update under ncu (65,536 cells of the benchmark
-# field, 16 passes: 367 MB + 412 MB), per cell and pass; scaled to a launch by cells x passes run
-UPDATE_DRAM_PER_CELL_PASS = (367.4e6 + 412.3e6) / (65536 * 16)
+# field, 16 passes: 558 MB + 422 MB), per cell and pass; scaled to a launch by cells x passes run
+UPDATE_DRAM_PER_CELL_PASS = (557.5e6 + 421.8e6) / (65536 * 16)
 
 
 def roofline(kt, n, passes_run, pk, flops_per_cell_pass, fp64_peak):
